@@ -10,13 +10,14 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 REPO = os.path.dirname(HERE)
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libbld.so")
-SOURCES = [os.path.join(HERE, "csrc", "bld_capi.cu")]
-DEPS = SOURCES + sorted(glob.glob(os.path.join(HERE, "csrc", "*.cuh"))) + [
+SOURCES = sorted(glob.glob(os.path.join(HERE, "csrc", "*.cu")))
+DEPS = SOURCES + sorted(glob.glob(os.path.join(HERE, "csrc", "*.cuh")) + glob.glob(os.path.join(HERE, "csrc", "*.h"))) + [
     os.path.join(REPO, "include", "bld.h")]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -39,12 +40,22 @@ def build(force=False, verbose=False, extra=()):
     if not force and up_to_date():
         return LIB
     os.makedirs(LIB_DIR, exist_ok=True)
-    cmd = [nvcc(), *ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-shared",
-           "-I", os.path.join(REPO, "include"), "-I", os.path.join(HERE, "csrc"),
-           "-o", LIB + ".tmp", *SOURCES, "-cudart", "static", *extra]
-    if verbose:
-        print(" ".join(cmd))
-    subprocess.run(cmd, check=True)
+    # one nvcc per source side by side, then the link
+    flags = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
+             "-I", os.path.join(REPO, "include"), "-I", os.path.join(HERE, "csrc"), *extra]
+    with tempfile.TemporaryDirectory() as tmp:
+        jobs = []
+        for src in SOURCES:
+            obj = os.path.join(tmp, os.path.basename(src) + ".o")
+            cmd = [nvcc(), *flags, "-c", "-o", obj, src]
+            if verbose:
+                print(" ".join(cmd))
+            jobs.append((cmd, obj, subprocess.Popen(cmd)))
+        failed = [cmd for cmd, _, p in jobs if p.wait() != 0]
+        if failed:
+            raise subprocess.CalledProcessError(1, failed[0])
+        subprocess.run([nvcc(), *ARCH, "-shared", "-o", LIB + ".tmp", *[o for _, o, _ in jobs], "-cudart", "static"],
+                       check=True)
     os.replace(LIB + ".tmp", LIB)
     return LIB
 

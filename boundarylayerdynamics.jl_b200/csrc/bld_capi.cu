@@ -3,36 +3,22 @@
 // kernel launch schedules per RK stage and CUDA-graph replay of whole steps.
 #include <cuda_runtime.h>
 
-#include <algorithm>
-#include <cmath>
 #include <cstdarg>
-#include <cstdio>
-#include <cstdlib>
-#include <cstdint>
-#include <cstring>
-#include <map>
-#include <mutex>
 #include <functional>
-#include <string>
+#include <mutex>
 #include <tuple>
-#include <initializer_list>
-#include <vector>
 
-#include "bld.h"
-#include "bld_kernels.cuh"
-#include "bld_warpx.cuh"
-#include "bld_advx2.cuh"
+#include "bld_engine.h"
 #include "bld_project_tile.cuh"
-#include "bld_sgsx2.cuh"
 
 double2 h_wtab64[BLD_WTAB_SIZE];
 float2 h_wtab32[BLD_WTAB_SIZE];
 
 namespace {
-
 thread_local std::string g_last_error;
+}
 
-int fail(int code, const char* fmt, ...) {
+int bld::fail(int code, const char* fmt, ...) {
     char buf[512];
     va_list ap;
     va_start(ap, fmt);
@@ -42,429 +28,7 @@ int fail(int code, const char* fmt, ...) {
     return code;
 }
 
-#define CUDA_TRY(expr)                                                                      \
-    do {                                                                                    \
-        cudaError_t e_ = (expr);                                                            \
-        if (e_ != cudaSuccess)                                                              \
-            return fail(e_ == cudaErrorMemoryAllocation ? BLD_ERR_OUT_OF_MEMORY : BLD_ERR_CUDA, \
-                        "%s: %s (%s:%d)", #expr, cudaGetErrorString(e_), __FILE__, __LINE__);  \
-    } while (0)
-
-#define BLD_TRY(expr)          \
-    do {                       \
-        int s_ = (expr);       \
-        if (s_ != BLD_OK) return s_; \
-    } while (0)
-
-// ---------------------------------------------------------------- FFT sizes and plans
-bool smooth_of(int n, std::initializer_list<int> primes) {
-    if (n < 2) return false;
-    for (int p : primes)
-        while (n % p == 0) n /= p;
-    return n == 1;
-}
-bool smooth23(int n) { return smooth_of(n, {2, 3}); }
-// sizes the block Stockham kernels transform: products of 2, 3, 5 and 7
-bool smooth2357(int n) { return smooth_of(n, {2, 3, 5, 7}); }
-
-int next_even_smooth(int n) {
-    int m = std::max(n, 2);
-    while (!(m % 2 == 0 && smooth23(m))) ++m;
-    return m;
-}
-
-// Fewest Stockham stages whose radices are register codelet sizes, then the
-// smallest largest radix (register pressure), capped at BLD_FP32_MAXR / BLD_FP64_MAXR;
-// nst = 0 if no such plan of at most four stages exists.
-FftPlan make_plan(int n, bool fp32 = false) {
-    static const int rads[] = {32, 24, 18, 16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
-    const int cap = fp32 ? BLD_FP32_MAXR : BLD_FP64_MAXR;
-    FftPlan best{};
-    best.n = n;
-    best.nst = 0;
-    int best_st = 99, best_max = 99;
-    int seq[6];
-    // depth-first search over radix sequences (n <= 1024 of 2, 3, 5, 7 needs at most 4 stages of <= 18)
-    auto dfs = [&](auto&& self, int rem, int depth, int mx) -> void {
-        if (depth > 4 || depth > best_st) return;
-        if (rem == 1) {
-            if (depth < best_st || (depth == best_st && mx < best_max)) {
-                best_st = depth;
-                best_max = mx;
-                best.nst = depth;
-                for (int i = 0; i < depth; ++i) best.radix[i] = seq[i];
-            }
-            return;
-        }
-        for (int r : rads) {
-            if (r > cap || rem % r) continue;
-            seq[depth] = r;
-            self(self, rem / r, depth + 1, std::max(mx, r));
-        }
-    };
-    dfs(dfs, n, 0, 0);
-    return best;
-}
-
-// quadratic-dealiasing size of the reference (src/physical_space.jl:49-56)
-int pdsize_quadratic(int kmax) {
-    const double l = std::log2(1.0 + kmax);
-    if (l == std::floor(l)) return 3 * kmax + 3;
-    return 3 * kmax + ((kmax % 2 == 1) ? 1 : 2);
-}
-
-struct DevTw {
-    void* d64 = nullptr;
-    void* d32 = nullptr;
-};
-
-// a y-pass variant: per-term (per-field) blocks with a two-buffer FFT, or one
-// block for all terms (fields) of a layer with an in-place FFT
-struct YCfg {
-    int all = 0;
-    int NL = 4;    // k1 lines per term (per field and line set)
-    int thr = 256;
-    int wfft = 0;  // per-term kernels: radix of the warp transform (P2 = 32 wfft), 0 = block stages
-    int tp = 0;    // 1: two-pass kernels (k_inv_y2 / k_fwd_y2), BLD_Y2_NL lines, P2 = A * B;
-                   // 2: inverse pass with TMA-staged tiles (k_inv_y3), BLD_Y3_NL lines;
-                   // 3: two-pass kernels on 8 lines (forward: 3 blocks per SM, 4 outputs in flight;
-                   //    inverse: 3 blocks per SM in double, 4 in single precision);
-                   // 4: forward two-pass kernel, single precision, 2 outputs in flight
-    int zc = 1;    // tp 2: layer chunks (blocks along z)
-};
-
-// radices of the warp y transforms compiled for the per-term y kernels
-// (24 in single precision only)
-bool wfft_radix_ok(int r, bool fp32) {
-    return r == 2 || r == 3 || r == 4 || r == 6 || r == 8 || r == 9 || r == 12 || r == 16 || (fp32 && r == 24);
-}
-
-struct Space {
-    bool on = false;
-    int P1 = 0, P2 = 0, ref_P1 = 0, ref_P2 = 0;
-    FftPlan plan1{}, plan2{};
-    int ntin = 0, ntout = 0;
-    void* min = nullptr;
-    void* mout = nullptr;
-    long long min_ms = 0, mout_ms = 0;  // elements per member
-    int YT = 1, PPT = 1, zchunk = 1, nchunks = 1;  // x kernels: rows per block, points per thread, z chunks
-    int xw = 0;                                     // > 0: warp-per-row x kernel with xw warps per block
-    int xwmb = 1;                                   // warp-per-row kernel: register cap (min blocks of 128 threads)
-    int zmult = 2;                                  // x kernels: z-chunk count multiplier in halves (autotuned)
-    int xb = 0;                                     // block of warps per row (advection): 1 three warps, 2 five (pipelined)
-    int x2 = 0;                                     // 1 + V: two-pass shared-memory x kernel k_adv_x2<.., V> (advection)
-    int sx2 = 0;                                    // SGS block x kernel with two-pass line transforms: 1 plain,
-                                                    // 2 registers capped for two blocks of 256 threads per SM,
-                                                    // 3 / 4 as 1 / 2 with the input rows staged by bulk copies
-    int sxk = 0;                                    // 1 + V: SGS x kernel k_sgs_x2<.., V> (rows staged by bulk copies, two-pass lines)
-    int xr = 0;                                     // block x kernels: warp-transform radix (P1 = 32 xr), 0 = Stockham
-    int fsets = 1;                                  // forward line sets (2 when a D2 contribution exists)
-    YCfg inv, fwd;                                  // y-pass variants (chosen by the autotuner)
-};
-
-}  // namespace
-
-struct bld_handle {
-    bld_config cfg{};
-    int device = 0;
-    int B = 1;
-    Geo g{};
-    bool fp32 = false;
-    cudaStream_t stream = nullptr;
-    // state and integrator buffers [member][vel1|vel2|vel3]
-    double2* u = nullptr;
-    double2* t = nullptr;
-    double2* du = nullptr;
-    double2* dp = nullptr;
-    double2* io = nullptr;     // staging for host-buffer calls
-    double2* io2 = nullptr;
-    double2* pscr = nullptr;
-    double* gamma = nullptr;
-    // tables
-    double *d1 = nullptr, *d2 = nullptr, *DD1 = nullptr, *DD2 = nullptr;
-    double *alpha_c = nullptr, *alpha_i = nullptr, *alpha_ext = nullptr, *mean_w = nullptr;
-    double* inv_alpha_c = nullptr;   // 1 / alpha_c (the projections' divergence)
-    double *lc2 = nullptr, *li2 = nullptr, *wall = nullptr, *src = nullptr, *mean_val = nullptr;
-    int* flag = nullptr;
-    int* flag_host = nullptr;
-    std::vector<int> diverged;   // members whose rates turned non-finite since the last bld_get_diverged
-    int* active = nullptr;        // [members] device mask of active ensemble slots
-    std::vector<int> active_host;
-    bool mask_on = false;        // the active mask applies to whole-ensemble steps only
-    int proj_variant = 1;        // 0: column kernel, 1/2: z-segmented kernel, 3: with a shared tile (autotuned)
-    int proj_tile = 0;           // LN > 0: projections of stored stage values by k_project_tile<.., LN> (autotuned)
-    int proj_pipe = 0;           // 1: ... by its persistent two-stage form k_project_pipe<.., LN> (autotuned)
-    double* prof_acc = nullptr;  // [members][3][n3+1] time integral of the mean profiles
-    double* prof_prev = nullptr; // [members][3][n3+1] last sample
-    bool prof_on = false;        // step graphs sample the profiles after every step
-    std::vector<double> tab_dx3c, tab_dx3i, tab_x3c, tab_x3i;  // copies of the mapping tables
-    std::vector<double> member_cs, member_z0;                  // current per-member SGS parameters
-    std::map<int, DevTw> tw;
-    Space adv, sgs;
-    // physical-domain transforms at the default size
-    int Pd1 = 0, Pd2 = 0;
-    void* pd_buf = nullptr;     // double [nz][Pd2][Pd1]
-    void* pd_mixed = nullptr;   // double2 [nz][Pd2][K1]
-    // progress statistics (allocated by the first bld_progress_stats call)
-    double* prog_small = nullptr;  // per-layer sums and maxima
-    void* prog_buf = nullptr;      // double [n3][P2][P1] at the largest physical size
-    void* prog_mixed = nullptr;    // double2 [n3][P2][K1]
-    // host-side copies used by launches
-    double w_lo = 0, w_hi = 0;
-    int dyn_lo = 0, dyn_hi = 0;
-    Linear lin{};
-    bool slope_valid = false;
-    bool ab2_started = false;
-    double ab2_dt = 0;
-    std::map<std::pair<int, double>, cudaGraphExec_t> graphs;
-    std::map<std::pair<int, double>, cudaGraph_t> graph_src;   // kept for ensemble parent graphs
-    std::map<std::vector<const void*>, cudaGraphExec_t> ens_graphs;  // parent graphs led by this handle
-    size_t bytes = 0;
-};
-
 namespace {
-
-int dalloc(bld_handle* h, void** p, size_t bytes) {
-    if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) return fail(BLD_ERR_OUT_OF_MEMORY, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
-    h->bytes += bytes;
-    return BLD_OK;
-}
-
-template <typename T>
-int upload(bld_handle* h, T** dst, const std::vector<T>& v) {
-    BLD_TRY(dalloc(h, (void**)dst, v.size() * sizeof(T)));
-    if (!v.empty()) CUDA_TRY(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return BLD_OK;
-}
-
-int twiddles(bld_handle* h, int n) {
-    if (h->tw.count(n)) return BLD_OK;
-    std::vector<double2> w64(n);
-    std::vector<float2> w32(n);
-    for (int m = 0; m < n; ++m) {
-        const long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)m / (long double)n;
-        const long double c = cosl(ang), s = sinl(ang);
-        w64[m] = make_double2((double)c, (double)s);
-        w32[m] = make_float2((float)c, (float)s);
-    }
-    DevTw t;
-    BLD_TRY(dalloc(h, &t.d64, n * sizeof(double2)));
-    BLD_TRY(dalloc(h, &t.d32, n * sizeof(float2)));
-    CUDA_TRY(cudaMemcpy(t.d64, w64.data(), n * sizeof(double2), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(t.d32, w32.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
-    h->tw[n] = t;
-    return BLD_OK;
-}
-
-const void* twp(const bld_handle* h, int n, bool fp32) {
-    const DevTw& t = h->tw.at(n);
-    return fp32 ? t.d32 : t.d64;
-}
-
-size_t csize(bool fp32) { return fp32 ? sizeof(float2) : sizeof(double2); }
-
-// y-pass lines per block: shared memory <= ~100 KB and outputs per thread <= 16
-// y-pass lines per block: the largest of 16 (single) / 8, 4, 2 whose two
-// shared line buffers (times `sets`) and twiddles stay within ~110 KB
-int pick_y(int P2, bool fp32, int sets) {
-    const size_t cs = csize(fp32);
-    int NL = fp32 ? 16 : 8;
-    while (NL > 2 && (size_t)(P2 + 2 * P2 * sets * NL) * cs > 110 * 1024) NL /= 2;
-    return NL;
-}
-
-// choose tiles for a physical-domain space
-// z chunks of the x kernels for the current rows per block: enough blocks to
-// fill the GPU a few times over, at least 8 layers per chunk
-void x_chunks(const bld_handle* h, Space& s) {
-    const int n3 = h->g.n3;
-    const int rows = s.x2 ? x2_rows((int)csize(h->fp32), s.P1, s.x2 - 1)
-                           : (s.sxk ? sx2_rows((int)csize(h->fp32), s.P1, s.sxk - 1) : (s.xb ? 1 : (s.xw ? s.xw : s.YT)));
-    const long long blocks_per_chunk = (long long)((s.P2 + rows - 1) / rows) * h->B;
-    int want = (int)std::max<long long>(1, (900 + blocks_per_chunk - 1) / blocks_per_chunk);
-    want = std::min(want, std::max(1, n3 / 8));
-    // the autotuner may ask for more chunks (shorter streams, more blocks: a
-    // smaller partial last wave), down to 4 layers per chunk
-    want = std::min(std::max(1, want * s.zmult / 2), std::max(1, n3 / 4));
-    s.zchunk = (n3 + want - 1) / want;
-    s.nchunks = (n3 + s.zchunk - 1) / s.zchunk;
-}
-
-// (rows per block, points per thread) candidates of the x kernels: blocks of
-// 32..256 threads whose two line buffers fit in 150 KB of shared memory
-std::vector<std::pair<int, int>> x_candidates(const bld_handle* h, const Space& s, bool is_adv) {
-    std::vector<std::pair<int, int>> out;
-    const int lines = is_adv ? 3 : 5;
-    for (int yt : {1, 2, 4}) {
-        if (s.P2 % yt || yt * s.P1 > 1024) continue;
-        if ((size_t)(s.P1 + 2 * lines * yt * s.P1) * csize(h->fp32) > 150 * 1024) continue;
-        for (int ppt = 1; ppt <= 4; ++ppt) {
-            const int pts = yt * s.P1;
-            if (pts % ppt) continue;
-            const int thr = pts / ppt;
-            if (thr > 256 || thr < 32) continue;
-            out.emplace_back(yt, ppt);
-        }
-    }
-    return out;
-}
-
-void tile_space(const bld_handle* h, Space& s, bool is_adv) {
-    // initial choice near 96 (advection, double) / 128 (SGS, double) / 192 (single)
-    // threads; the autotuner replaces it with the measured best
-    const int target = h->fp32 ? 192 : (is_adv ? 96 : 128);
-    int best = 1 << 30;
-    s.YT = 1;
-    s.PPT = 0;
-    for (auto c : x_candidates(h, s, is_adv)) {
-        const int thr = c.first * s.P1 / c.second;
-        const int score = std::abs(thr - target) + 24 * (c.second - 1) + 8 * (c.first - 1);
-        if (score < best) {
-            best = score;
-            s.YT = c.first;
-            s.PPT = c.second;
-        }
-    }
-    x_chunks(h, s);
-}
-
-size_t smem_y(int P2, int NL, bool fp32) { return (size_t)(P2 + 2 * P2 * NL) * csize(fp32); }
-// per-term y kernels with `lines` lines: twiddles and two line buffers for the
-// block-wide stages, or twiddles and one buffer of P2 + 32 (swizzled) positions
-// on a line stride of lines + 1 for the warp transforms
-size_t smem_y_term(int P2, int lines, int wfft, bool fp32) {
-    return (size_t)(wfft ? P2 + (P2 + 32) * (lines + 1) : P2 + 2 * P2 * lines) * csize(fp32);
-}
-// block x kernels: twiddles and two buffers of (3 or 5) YT lines, on a line stride
-// P1 + 32 (swizzled positions) with warp line transforms (xr > 0)
-size_t smem_adv(const Space& s, bool fp32) {
-    return (size_t)(s.P1 + 2 * 3 * s.YT * (s.P1 + (s.xr ? 32 : 0))) * csize(fp32);
-}
-// the two-pass SGS kernel stages its input rows by bulk copies when a block's
-// YT rows of K1 values fill whole 16-byte units
-bool sgs_stage_fits(const Space& s, bool fp32, int K1) { return !fp32 || K1 % 2 == 0 || s.YT % 2 == 0; }
-bool sgs_staged(const Space& s, bool fp32, int K1) { return s.sx2 >= 3 && sgs_stage_fits(s, fp32, K1); }
-
-size_t smem_sgs(const Space& s, bool fp32, int K1) {
-    if (s.sx2) {
-        const int A = y2_radix_a(s.P1), B = y2_radix_b(s.P1);
-        const int lp = fp32 ? twopass_line<float2>(A, B) : twopass_line<double2>(A, B);
-        if (sgs_staged(s, fp32, K1))
-            return (size_t)sgs_stage_offset(s.P1, 5 * s.YT, lp, (int)csize(fp32)) + 128 +
-                   (size_t)2 * 9 * s.YT * K1 * csize(fp32);
-        return (size_t)(s.P1 + 2 * 5 * s.YT * lp) * csize(fp32);
-    }
-    return (size_t)(s.P1 + 2 * 5 * s.YT * (s.P1 + (s.xr ? 32 : 0))) * csize(fp32);
-}
-
-// ------------------------------------------------------------------ kernel dispatch
-// threads for an in-place transform of `lines` lines (one task per thread for
-// radix >= 8, up to four for smaller radices); 0 if more than 384 are needed
-int inplace_threads(const FftPlan& pl, int lines) {
-    int thr = 32;
-    for (int i = 0; i < pl.nst; ++i) {
-        const int r = pl.radix[i];
-        const int tpt = r <= 4 ? 4 : (r == 6 ? 3 : 1);  // inplace_tpt
-        const int tasks = lines * pl.n / r;
-        thr = std::max(thr, (tasks + tpt - 1) / tpt);
-    }
-    thr = (thr + 31) / 32 * 32;
-    return thr <= 384 ? thr : 0;
-}
-
-// threads of a y-pass block: enough for the widest FFT stage of `lines` lines
-int y_threads(const FftPlan& pl, int lines) {
-    int rmin = 64;
-    for (int i = 0; i < pl.nst; ++i) rmin = std::min(rmin, pl.radix[i]);
-    const int tasks = lines * pl.n / rmin;
-    return std::min(256, std::max(64, (tasks + 31) / 32 * 32));
-}
-
-// two-pass y kernels: compiled for P2 with a factorisation y2_radix_a/b (single
-// precision up to 768, double up to 288) and their registers per block count
-bool y2_ok(int P2, bool fp32) { return y2_radix_a(P2) > 0 && (fp32 || P2 <= 288); }
-size_t smem_y2(int P2, int lines, bool fp32) { return (size_t)P2 * (1 + lines) * csize(fp32); }
-
-template <typename R, int P>
-int launch_y2_p(bld_handle* h, bool inverse, const void* args, dim3 grid, size_t sm, int tp) {
-    constexpr int A = y2_radix_a(P), B = y2_radix_b(P);
-    constexpr int MINB = y2_min_blocks<R>(B * BLD_Y2_NL);
-    constexpr int MINBI = y2_min_blocks_inv<R>(B * BLD_Y2_NL);
-    if (!inverse && tp == 3)
-        k_fwd_y2<R, A, B, 3, 8, 4><<<grid, B * 8, sm, h->stream>>>(*static_cast<const FwdYArgs*>(args));
-    else if (inverse && tp == 3)   // eight lines: three (double) or four (single precision) blocks per SM
-        k_inv_y2<R, A, B, sizeof(R) == 8 ? 3 : 4, 8><<<grid, B * 8, sm, h->stream>>>(
-            *static_cast<const InvYArgs*>(args));
-    else if (!inverse && tp == 4 && sizeof(R) == 4)
-        k_fwd_y2<R, A, B, MINB, BLD_Y2_NL, 2><<<grid, B * BLD_Y2_NL, sm, h->stream>>>(
-            *static_cast<const FwdYArgs*>(args));
-    else if (inverse)
-        k_inv_y2<R, A, B, MINBI><<<grid, B * BLD_Y2_NL, sm, h->stream>>>(*static_cast<const InvYArgs*>(args));
-    else
-        k_fwd_y2<R, A, B, MINB><<<grid, B * BLD_Y2_NL, sm, h->stream>>>(*static_cast<const FwdYArgs*>(args));
-    return BLD_OK;
-}
-
-template <typename R>
-int launch_y2(bld_handle* h, int P2, bool inverse, const void* args, dim3 grid, size_t sm, int tp = 1) {
-    switch (P2) {
-        case 64: return launch_y2_p<R, 64>(h, inverse, args, grid, sm, tp);
-        case 96: return launch_y2_p<R, 96>(h, inverse, args, grid, sm, tp);
-        case 128: return launch_y2_p<R, 128>(h, inverse, args, grid, sm, tp);
-        case 144: return launch_y2_p<R, 144>(h, inverse, args, grid, sm, tp);
-        case 192: return launch_y2_p<R, 192>(h, inverse, args, grid, sm, tp);
-        case 256: return launch_y2_p<R, 256>(h, inverse, args, grid, sm, tp);
-        case 288: return launch_y2_p<R, 288>(h, inverse, args, grid, sm, tp);
-        default: break;
-    }
-    if constexpr (sizeof(R) == 4) {
-        switch (P2) {
-            case 384: return launch_y2_p<R, 384>(h, inverse, args, grid, sm, tp);
-            case 512: return launch_y2_p<R, 512>(h, inverse, args, grid, sm, tp);
-            case 768: return launch_y2_p<R, 768>(h, inverse, args, grid, sm, tp);
-            default: break;
-        }
-    }
-    return fail(BLD_ERR_INVALID_CONFIG, "no two-pass y transform for P2=%d", P2);
-}
-
-// cuTensorMapEncodeTiled from the driver, found through the runtime (the
-// library links only the static CUDA runtime)
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
-}
-
-// the members' states from `base` as a float64 tensor (2 K1, K2, 3 n3 - 1, members)
-// with the box (2 NL, K2, 1, 1) of k_inv_y3
-int state_tmap(const bld_handle* h, const void* base, int nl, CUtensorMap* out) {
-    const Geo& g = h->g;
-    EncodeTiledFn fn = encode_tiled();
-    if (!fn) return fail(BLD_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-    const cuuint64_t dims[4] = {(cuuint64_t)(2 * g.K1), (cuuint64_t)g.K2, (cuuint64_t)(3 * g.n3 - 1), (cuuint64_t)h->B};
-    const cuuint64_t strides[3] = {(cuuint64_t)g.K1 * 16, (cuuint64_t)g.F * 16, (cuuint64_t)g.mstride * 16};
-    const cuuint32_t box[4] = {(cuuint32_t)(2 * nl), (cuuint32_t)g.K2, 1, 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(base), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(BLD_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-    return BLD_OK;
-}
 
 // k_project_tile applies: the pressure solve with <= 256 layers, an even number
 // of modes per layer (gamma rows are 16-byte multiples for the TMA map) and
@@ -535,637 +99,25 @@ int project_tmaps(const bld_handle* h, const void* u, int ln, CUtensorMap* umap,
     return BLD_OK;
 }
 
-// k_inv_y3 applies: a two-pass factorisation, whole K2 columns in one TMA box
-// (K2 <= 256) and the staged tiles within the shared memory of a block
-bool y3_ok(const bld_handle* h, int P2) {
-    return y2_ok(P2, h->fp32) && h->g.K2 <= 256 &&
-           y3_smem(P2, h->g.K2, (int)csize(h->fp32)) <= 227 * 1024 && encode_tiled() != nullptr;
+// The in-place x kernels: compiled for the sizes of bld_xrow.h.  Advection needs the
+// 3/2 rule's empty middle third where P1 is a multiple of 3, the Smagorinsky kernel the
+// default grid P1 = 2 k1max + 2.  The switches that ask for another family keep them
+// out.
+bool row_ok(const bld_handle* h, int P1, int P2, bool is_adv) {
+    for (const char* v : {"BLD_X_KERNEL", "BLD_X_LINES", is_adv ? "BLD_X2_VARIANT" : "BLD_SGS_X_KERNEL",
+                          is_adv ? "BLD_XW_MINB" : "BLD_SGS_X2_VARIANT"}) {
+        const char* e = getenv(v);
+        if (e && e[0] && strcmp(e, "inplace")) return false;
+    }
+    const bld_row::Shape r = is_adv ? bld_row::adv_shape(P1, h->fp32) : bld_row::sgs_shape(P1, h->fp32);
+    if (!(is_adv ? bld_row::adv_compiled(P1, h->fp32) : bld_row::sgs_compiled(P1, h->fp32)) || P2 % r.NR) return false;
+    return is_adv ? P1 % 3 != 0 || 3 * h->g.k1max < P1 : P1 == 2 * h->g.k1max + 2;
 }
-
-template <typename R, int P>
-int launch_y3_p(bld_handle* h, const InvYArgs& a, const CUtensorMap& map, dim3 grid) {
-    constexpr int A = y2_radix_a(P), B = y2_radix_b(P);
-    const size_t sm = y3_smem(P, h->g.K2, (int)sizeof(cplx<R>));
-    k_inv_y3<R, A, B><<<grid, B * BLD_Y3_NL, sm, h->stream>>>(a, map);
-    return BLD_OK;
-}
-
-template <typename R>
-int launch_inv_y3(bld_handle* h, const Space& s, InvYArgs a, int nm) {
-    CUtensorMap map;
-    BLD_TRY(state_tmap(h, a.state, BLD_Y3_NL, &map));
-    a.NL = BLD_Y3_NL;
-    a.zchunk = (h->g.n3 + s.inv.zc - 1) / s.inv.zc;
-    a.flag = h->flag;
-    dim3 grid(a.nterms * nm, (h->g.K1 + BLD_Y3_NL - 1) / BLD_Y3_NL, (h->g.n3 + a.zchunk - 1) / a.zchunk);
-    switch (s.P2) {
-        case 64: return launch_y3_p<R, 64>(h, a, map, grid);
-        case 96: return launch_y3_p<R, 96>(h, a, map, grid);
-        case 128: return launch_y3_p<R, 128>(h, a, map, grid);
-        case 144: return launch_y3_p<R, 144>(h, a, map, grid);
-        case 192: return launch_y3_p<R, 192>(h, a, map, grid);
-        case 256: return launch_y3_p<R, 256>(h, a, map, grid);
-        case 288: return launch_y3_p<R, 288>(h, a, map, grid);
-        default: break;
-    }
-    if constexpr (sizeof(R) == 4) {
-        switch (s.P2) {
-            case 384: return launch_y3_p<R, 384>(h, a, map, grid);
-            case 512: return launch_y3_p<R, 512>(h, a, map, grid);
-            case 768: return launch_y3_p<R, 768>(h, a, map, grid);
-            default: break;
-        }
-    }
-    return fail(BLD_ERR_INVALID_CONFIG, "no TMA y transform for P2=%d", s.P2);
-}
-
-template <typename R>
-int launch_inv_y(bld_handle* h, const Space& s, InvYArgs a, int nm) {
-    const YCfg& c = s.inv;
-    a.NL = c.NL;
-    const size_t cs = csize(sizeof(R) == 4);
-    if (c.tp == 2) {
-        BLD_TRY(launch_inv_y3<R>(h, s, a, nm));
-        CUDA_TRY(cudaGetLastError());
-        return BLD_OK;
-    }
-    if (c.tp) {
-        const int nl = c.tp == 3 ? 8 : BLD_Y2_NL;
-        a.NL = nl;
-        dim3 grid(a.nterms * nm, (h->g.K1 + nl - 1) / nl, h->g.n3);
-        BLD_TRY(launch_y2<R>(h, s.P2, true, &a, grid, smem_y2(s.P2, nl, sizeof(R) == 4), c.tp));
-        CUDA_TRY(cudaGetLastError());
-        return BLD_OK;
-    }
-    if (c.all) {
-        dim3 grid((h->g.K1 + c.NL - 1) / c.NL, h->g.n3, nm);
-        k_inv_y_all<R><<<grid, c.thr, (size_t)(s.P2 + s.P2 * a.nterms * c.NL) * cs, h->stream>>>(a);
-    } else {
-        dim3 grid(a.nterms * nm, (h->g.K1 + c.NL - 1) / c.NL, h->g.n3);
-        const size_t sm = smem_y_term(s.P2, c.NL, c.wfft, sizeof(R) == 4);
-        switch (c.wfft) {
-            case 0: k_inv_y<R, 0><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 2: k_inv_y<R, 2><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 3: k_inv_y<R, 3><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 4: k_inv_y<R, 4><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 6: k_inv_y<R, 6><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 8: k_inv_y<R, 8><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 9: k_inv_y<R, 9><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 12: k_inv_y<R, 12><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 16: k_inv_y<R, 16><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 24:
-                if constexpr (sizeof(R) == 4) {
-                    k_inv_y<R, 24><<<grid, c.thr, sm, h->stream>>>(a);
-                    break;
-                }
-                return fail(BLD_ERR_INVALID_CONFIG, "no warp y transform of radix %d", c.wfft);
-            default: return fail(BLD_ERR_INVALID_CONFIG, "no warp y transform of radix %d", c.wfft);
-        }
-    }
-    CUDA_TRY(cudaGetLastError());
-    return BLD_OK;
-}
-
-template <typename R>
-int launch_fwd_y(bld_handle* h, const Space& s, FwdYArgs a, int nm) {
-    const YCfg& c = s.fwd;
-    a.NL = c.NL;
-    const size_t cs = csize(sizeof(R) == 4);
-    if (c.tp) {
-        const int nl = c.tp == 3 ? 8 : BLD_Y2_NL;   // tp 1, 2, 4: BLD_Y2_NL lines
-        a.NL = nl;
-        dim3 grid(a.fields * nm, (h->g.K1 + nl - 1) / nl, h->g.n3);
-        BLD_TRY(launch_y2<R>(h, s.P2, false, &a, grid, smem_y2(s.P2, s.fsets * nl, sizeof(R) == 4), c.tp));
-        CUDA_TRY(cudaGetLastError());
-        return BLD_OK;
-    }
-    if (c.all) {
-        dim3 grid((h->g.K1 + c.NL - 1) / c.NL, h->g.n3, nm);
-        k_fwd_y_all<R><<<grid, c.thr, (size_t)(s.P2 + s.P2 * 3 * s.fsets * c.NL) * cs, h->stream>>>(a);
-    } else {
-        dim3 grid(a.fields * nm, (h->g.K1 + c.NL - 1) / c.NL, h->g.n3);
-        const size_t sm = smem_y_term(s.P2, s.fsets * c.NL, c.wfft, sizeof(R) == 4);
-        switch (c.wfft) {
-            case 0: k_fwd_y<R, 0><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 2: k_fwd_y<R, 2><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 3: k_fwd_y<R, 3><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 4: k_fwd_y<R, 4><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 6: k_fwd_y<R, 6><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 8: k_fwd_y<R, 8><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 9: k_fwd_y<R, 9><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 12: k_fwd_y<R, 12><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 16: k_fwd_y<R, 16><<<grid, c.thr, sm, h->stream>>>(a); break;
-            case 24:
-                if constexpr (sizeof(R) == 4) {
-                    k_fwd_y<R, 24><<<grid, c.thr, sm, h->stream>>>(a);
-                    break;
-                }
-                return fail(BLD_ERR_INVALID_CONFIG, "no warp y transform of radix %d", c.wfft);
-            default: return fail(BLD_ERR_INVALID_CONFIG, "no warp y transform of radix %d", c.wfft);
-        }
-    }
-    CUDA_TRY(cudaGetLastError());
-    return BLD_OK;
-}
-
-// two-pass advection x kernel: compiled for P1 with a two-pass factorisation
-// (single precision up to 768, double up to 288), whole row pairs per block;
-// variants V = 2 (wide) in double precision, V = 3 (two rows) in single precision up to 384
-bool x2_ok(const bld_handle* h, const Space& s, int V = 0) {
-    const int cs = (int)csize(h->fp32);
-    return y2_ok(s.P1, h->fp32) && s.P2 % x2_rows(cs, s.P1, V) == 0 &&
-           (V == 0 || (V == 2 && !h->fp32) || (V == 3 && h->fp32 && s.P1 <= 384)) &&
-           x2_smem(y2_radix_a(s.P1), y2_radix_b(s.P1), h->g.K1, cs, V) <= 227 * 1024;
-}
-
-template <typename R, int P, int V>
-void launch_x2_pv(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    constexpr int A = y2_radix_a(P), B = y2_radix_b(P);
-    constexpr int NR = x2_rows((int)sizeof(cplx<R>), P, V);
-    dim3 grid(s.P2 / NR, s.nchunks, nm);
-    const size_t sm = x2_smem(A, B, h->g.K1, (int)sizeof(cplx<R>), V);
-    k_adv_x2<R, A, B, V><<<grid, x2_threads(B, NR, V), sm, h->stream>>>(a, h->flag);
-}
-
-template <typename R, int P>
-int launch_x2_p(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    if constexpr (sizeof(R) == 8) {
-        if (s.x2 == 3) return launch_x2_pv<R, P, 2>(h, s, a, nm), BLD_OK;
-    }
-    if constexpr (sizeof(R) == 4 && P <= 384) {
-        if (s.x2 == 4) return launch_x2_pv<R, P, 3>(h, s, a, nm), BLD_OK;
-    }
-    launch_x2_pv<R, P, 0>(h, s, a, nm);
-    return BLD_OK;
-}
-
-template <typename R>
-int launch_adv_x2(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    switch (s.P1) {
-        case 64: BLD_TRY((launch_x2_p<R, 64>(h, s, a, nm))); break;
-        case 96: BLD_TRY((launch_x2_p<R, 96>(h, s, a, nm))); break;
-        case 128: BLD_TRY((launch_x2_p<R, 128>(h, s, a, nm))); break;
-        case 144: BLD_TRY((launch_x2_p<R, 144>(h, s, a, nm))); break;
-        case 192: BLD_TRY((launch_x2_p<R, 192>(h, s, a, nm))); break;
-        case 256: BLD_TRY((launch_x2_p<R, 256>(h, s, a, nm))); break;
-        case 288: BLD_TRY((launch_x2_p<R, 288>(h, s, a, nm))); break;
-        default:
-            if constexpr (sizeof(R) == 4) {
-                if (s.P1 == 384) { BLD_TRY((launch_x2_p<R, 384>(h, s, a, nm))); break; }
-                if (s.P1 == 512) { BLD_TRY((launch_x2_p<R, 512>(h, s, a, nm))); break; }
-                if (s.P1 == 768) { BLD_TRY((launch_x2_p<R, 768>(h, s, a, nm))); break; }
-            }
-            return fail(BLD_ERR_INVALID_CONFIG, "no two-pass x kernel for P1=%d", s.P1);
-    }
-    CUDA_TRY(cudaGetLastError());
-    return BLD_OK;
-}
-
-// radices of the warp line transforms compiled into the block x kernels, and the
-// points per thread that go with each (so that YT * 32 RAD / PPT threads are whole warps)
-bool xr_radix_ok(int r) { return r == 2 || r == 3 || r == 4 || r == 6 || r == 8 || r == 9 || r == 12 || r == 16 || r == 24; }
-constexpr int xr_ppt(int r) { return r <= 4 ? 1 : r <= 8 ? 2 : r <= 12 ? 3 : 4; }
-
-#define BLD_XR_CASES(KERNEL)                                                                          \
-    case 2: KERNEL<R, xr_ppt(2), 2><<<grid, thr, sm, h->stream>>>(a); break;                         \
-    case 3: KERNEL<R, xr_ppt(3), 3><<<grid, thr, sm, h->stream>>>(a); break;                         \
-    case 4: KERNEL<R, xr_ppt(4), 4><<<grid, thr, sm, h->stream>>>(a); break;                         \
-    case 6: KERNEL<R, xr_ppt(6), 6><<<grid, thr, sm, h->stream>>>(a); break;                         \
-    case 8: KERNEL<R, xr_ppt(8), 8><<<grid, thr, sm, h->stream>>>(a); break;                         \
-    case 9: KERNEL<R, xr_ppt(9), 9><<<grid, thr, sm, h->stream>>>(a); break;                         \
-    case 12: KERNEL<R, xr_ppt(12), 12><<<grid, thr, sm, h->stream>>>(a); break;                      \
-    case 16: KERNEL<R, xr_ppt(16), 16><<<grid, thr, sm, h->stream>>>(a); break;                      \
-    case 24: KERNEL<R, xr_ppt(24), 24><<<grid, thr, sm, h->stream>>>(a); break;
-
-template <typename R>
-int launch_adv_x(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    dim3 grid(s.P2 / s.YT, s.nchunks, nm);
-    const int thr = s.YT * s.P1 / s.PPT;
-    const size_t sm = smem_adv(s, sizeof(R) == 4);
-    if (s.xr) {
-        switch (s.xr) {
-            BLD_XR_CASES(k_adv_x)
-            default: return fail(BLD_ERR_INVALID_CONFIG, "no warp x transform of radix %d", s.xr);
-        }
-    } else {
-        switch (s.PPT) {
-            case 1: k_adv_x<R, 1, 0><<<grid, thr, sm, h->stream>>>(a); break;
-            case 2: k_adv_x<R, 2, 0><<<grid, thr, sm, h->stream>>>(a); break;
-            case 3: k_adv_x<R, 3, 0><<<grid, thr, sm, h->stream>>>(a); break;
-            default: k_adv_x<R, 4, 0><<<grid, thr, sm, h->stream>>>(a); break;
-        }
-    }
-    CUDA_TRY(cudaGetLastError());
-    return BLD_OK;
-}
-
-// radix of the warp-per-row x kernel for P1 = 32 * radix, or 0 if no variant is compiled
-template <typename R>
-int warpx_radix(int P1) {
-    if (P1 % 32) return 0;
-    const int r = P1 / 32;
-    if (sizeof(R) == 8) return (r == 2 || r == 3 || r == 4 || r == 6) ? r : 0;
-    return (r == 2 || r == 3 || r == 4 || r == 6 || r == 8 || r == 9 || r == 12) ? r : 0;
-}
-
-// register caps compiled for the warp-per-row x kernel (single precision, radix >= 8)
-template <typename R>
-bool warpx_minb_ok(int r, int mb) {
-    if (mb == 1) return true;
-    return sizeof(R) == 4 && (r == 8 || r == 9 || r == 12) && (mb == 3 || mb == 4);
-}
-
-template <typename R>
-int launch_adv_xw(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    const int r = warpx_radix<R>(s.P1);
-    dim3 grid((s.P2 + s.xw - 1) / s.xw, s.nchunks, nm);
-    const int thr = 32 * s.xw;
-    const size_t sm = ((size_t)r * 32 + (size_t)s.xw * 12 * h->g.K1) * csize(sizeof(R) == 4);
-    if constexpr (sizeof(R) == 4) {
-        if (s.xwmb > 1) {
-            if (!warpx_minb_ok<R>(r, s.xwmb)) return fail(BLD_ERR_INVALID_CONFIG, "no capped warp x kernel");
-#define BLD_XW_MB(RR)                                                                   \
-    case RR:                                                                            \
-        if (s.xwmb == 3) k_adv_xwc<R, RR, 3><<<grid, thr, sm, h->stream>>>(a);          \
-        else k_adv_xwc<R, RR, 4><<<grid, thr, sm, h->stream>>>(a);                      \
-        break;
-            switch (r) {
-                BLD_XW_MB(8)
-                BLD_XW_MB(9)
-                BLD_XW_MB(12)
-                default: return fail(BLD_ERR_INVALID_CONFIG, "no capped warp x kernel");
-            }
-#undef BLD_XW_MB
-            CUDA_TRY(cudaGetLastError());
-            return BLD_OK;
-        }
-    }
-    switch (r) {
-        case 2: k_adv_xw<R, 2><<<grid, thr, sm, h->stream>>>(a); break;
-        case 3: k_adv_xw<R, 3><<<grid, thr, sm, h->stream>>>(a); break;
-        case 4: k_adv_xw<R, 4><<<grid, thr, sm, h->stream>>>(a); break;
-        case 6: k_adv_xw<R, 6><<<grid, thr, sm, h->stream>>>(a); break;
-        default:
-            if constexpr (sizeof(R) == 4) {
-                switch (r) {
-                    case 8: k_adv_xw<R, 8><<<grid, thr, sm, h->stream>>>(a); break;
-                    case 9: k_adv_xw<R, 9><<<grid, thr, sm, h->stream>>>(a); break;
-                    case 12: k_adv_xw<R, 12><<<grid, thr, sm, h->stream>>>(a); break;
-                    default: return fail(BLD_ERR_INVALID_CONFIG, "no warp x kernel for P1=%d", s.P1);
-                }
-            } else {
-                return fail(BLD_ERR_INVALID_CONFIG, "no warp x kernel for P1=%d", s.P1);
-            }
-    }
-    CUDA_TRY(cudaGetLastError());
-    return BLD_OK;
-}
-
-// radix of the block-of-warps x kernels for P1 = 32 * radix (16 and 24 in single
-// precision only: one line of 24 FP64 complex values per lane would spill), or 0
-int xb_radix(int P1, bool fp32) {
-    if (P1 % 32) return 0;
-    const int r = P1 / 32;
-    if (fp32 && (r == 16 || r == 24)) return r;
-    return (r == 2 || r == 3 || r == 4 || r == 6 || r == 8 || r == 9 || r == 12) ? r : 0;
-}
-
-template <typename R>
-int launch_adv_xb(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    const int r = xb_radix(s.P1, sizeof(R) == 4);
-    dim3 grid(s.P2, s.nchunks, nm);
-    if (s.xb == 2) {
-        const size_t smp = ((size_t)r * 32 + 5 * (size_t)(s.P1 + 32) + 12 * (size_t)h->g.K1) * csize(sizeof(R) == 4);
-        switch (r) {
-            case 2: k_adv_xp<R, 2><<<grid, 160, smp, h->stream>>>(a); break;
-            case 3: k_adv_xp<R, 3><<<grid, 160, smp, h->stream>>>(a); break;
-            case 4: k_adv_xp<R, 4><<<grid, 160, smp, h->stream>>>(a); break;
-            case 6: k_adv_xp<R, 6><<<grid, 160, smp, h->stream>>>(a); break;
-            case 8: k_adv_xp<R, 8><<<grid, 160, smp, h->stream>>>(a); break;
-            case 9: k_adv_xp<R, 9><<<grid, 160, smp, h->stream>>>(a); break;
-            case 12: k_adv_xp<R, 12><<<grid, 160, smp, h->stream>>>(a); break;
-            default:
-                if constexpr (sizeof(R) == 4) {
-                    if (r == 16) { k_adv_xp<R, 16><<<grid, 160, smp, h->stream>>>(a); break; }
-                    if (r == 24) { k_adv_xp<R, 24><<<grid, 160, smp, h->stream>>>(a); break; }
-                }
-                return fail(BLD_ERR_INVALID_CONFIG, "no pipelined block-of-warps x kernel for P1=%d", s.P1);
-        }
-        CUDA_TRY(cudaGetLastError());
-        return BLD_OK;
-    }
-    const size_t sm = ((size_t)r * 32 + 3 * (size_t)(s.P1 + 32) + 12 * (size_t)h->g.K1) * csize(sizeof(R) == 4);
-    switch (r) {
-        case 2: k_adv_xb<R, 2><<<grid, 96, sm, h->stream>>>(a); break;
-        case 3: k_adv_xb<R, 3><<<grid, 96, sm, h->stream>>>(a); break;
-        case 4: k_adv_xb<R, 4><<<grid, 96, sm, h->stream>>>(a); break;
-        case 6: k_adv_xb<R, 6><<<grid, 96, sm, h->stream>>>(a); break;
-        case 8: k_adv_xb<R, 8><<<grid, 96, sm, h->stream>>>(a); break;
-        case 9: k_adv_xb<R, 9><<<grid, 96, sm, h->stream>>>(a); break;
-        case 12: k_adv_xb<R, 12><<<grid, 96, sm, h->stream>>>(a); break;
-        default:
-            if constexpr (sizeof(R) == 4) {
-                if (r == 16) { k_adv_xb<R, 16><<<grid, 96, sm, h->stream>>>(a); break; }
-                if (r == 24) { k_adv_xb<R, 24><<<grid, 96, sm, h->stream>>>(a); break; }
-            }
-            return fail(BLD_ERR_INVALID_CONFIG, "no block-of-warps x kernel for P1=%d", s.P1);
-    }
-    CUDA_TRY(cudaGetLastError());
-    return BLD_OK;
-}
-
-// the register-capped two-pass SGS x kernels: single precision, P1 >= 256
-// (where the uncapped kernel needs ~170 registers, one block per SM)
-__host__ __device__ constexpr bool sx2_capped_size(int P) { return P >= 256; }
-
-template <typename R, int P>
-int launch_sgs_x2_p(bld_handle* h, const Space& s, const XArgs& a, dim3 grid, int thr, size_t sm) {
-    if constexpr (sizeof(R) == 4 && sx2_capped_size(P)) {
-        if (s.sx2 == 2 || s.sx2 == 4) {
-            if (s.PPT == 1)
-                k_sgs_x<R, 1, 0, P, 2><<<grid, thr, sm, h->stream>>>(a);
-            else
-                k_sgs_x<R, 2, 0, P, 2><<<grid, thr, sm, h->stream>>>(a);
-            return BLD_OK;
-        }
-    }
-    if (s.PPT == 1)
-        k_sgs_x<R, 1, 0, P><<<grid, thr, sm, h->stream>>>(a);
+int launch_row(bld_handle* h, const Space& s, const XArgs& a, int nm) {
+    if (&s == &h->adv)
+        CUDA_TRY((h->fp32 ? bld_row::launch_adv32 : bld_row::launch_adv64)(a, s.nchunks, nm, h->stream));
     else
-        k_sgs_x<R, 2, 0, P><<<grid, thr, sm, h->stream>>>(a);
-    return BLD_OK;
-}
-
-// SGS x kernel with two-pass line transforms: compiled for the two-pass sizes and
-// one or two points per thread of the products; v = 2: the register-capped form
-bool sx2_ok(const bld_handle* h, const Space& s, int v = 1) {
-    return y2_ok(s.P1, h->fp32) && (v % 2 == 1 || (h->fp32 && sx2_capped_size(s.P1)));
-}
-
-// k_sgs_x2: compiled for the two-pass sizes; whole row groups per block
-// V = 1 (two rows per block) in single precision up to P1 = 384
-bool sxk_ok(const bld_handle* h, const Space& s, int V = 0) {
-    const int cs = (int)csize(h->fp32);
-    return y2_ok(s.P1, h->fp32) && (V == 0 || (h->fp32 && s.P1 <= 384)) && s.P2 % sx2_rows(cs, s.P1, V) == 0 &&
-           sx2_smem(y2_radix_a(s.P1), y2_radix_b(s.P1), h->g.K1, cs, V) <= 227 * 1024;
-}
-
-template <typename R, int P, int V>
-void launch_sgs_xk_pv(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    constexpr int A = y2_radix_a(P), B = y2_radix_b(P);
-    constexpr int NR = sx2_rows((int)sizeof(cplx<R>), P, V);
-    dim3 grid(s.P2 / NR, s.nchunks, nm);
-    const size_t sm = sx2_smem(A, B, h->g.K1, (int)sizeof(cplx<R>), V);
-    k_sgs_x2<R, A, B, V><<<grid, sx2_threads(B, NR), sm, h->stream>>>(a);
-}
-
-template <typename R, int P>
-int launch_sgs_xk_p(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    if constexpr (sizeof(R) == 4 && P <= 384) {
-        if (s.sxk == 2) return launch_sgs_xk_pv<R, P, 1>(h, s, a, nm), BLD_OK;
-    }
-    launch_sgs_xk_pv<R, P, 0>(h, s, a, nm);
-    return BLD_OK;
-}
-
-template <typename R>
-int launch_sgs_xk(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    switch (s.P1) {
-        case 64: BLD_TRY((launch_sgs_xk_p<R, 64>(h, s, a, nm))); break;
-        case 96: BLD_TRY((launch_sgs_xk_p<R, 96>(h, s, a, nm))); break;
-        case 128: BLD_TRY((launch_sgs_xk_p<R, 128>(h, s, a, nm))); break;
-        case 144: BLD_TRY((launch_sgs_xk_p<R, 144>(h, s, a, nm))); break;
-        case 192: BLD_TRY((launch_sgs_xk_p<R, 192>(h, s, a, nm))); break;
-        case 256: BLD_TRY((launch_sgs_xk_p<R, 256>(h, s, a, nm))); break;
-        case 288: BLD_TRY((launch_sgs_xk_p<R, 288>(h, s, a, nm))); break;
-        default:
-            if constexpr (sizeof(R) == 4) {
-                if (s.P1 == 384) { BLD_TRY((launch_sgs_xk_p<R, 384>(h, s, a, nm))); break; }
-                if (s.P1 == 512) { BLD_TRY((launch_sgs_xk_p<R, 512>(h, s, a, nm))); break; }
-                if (s.P1 == 768) { BLD_TRY((launch_sgs_xk_p<R, 768>(h, s, a, nm))); break; }
-            }
-            return fail(BLD_ERR_INVALID_CONFIG, "no k_sgs_x2 kernel for P1=%d", s.P1);
-    }
-    CUDA_TRY(cudaGetLastError());
-    return BLD_OK;
-}
-
-template <typename R>
-int launch_sgs_x(bld_handle* h, const Space& s, const XArgs& a, int nm) {
-    if (s.sxk) return launch_sgs_xk<R>(h, s, a, nm);
-    dim3 grid(s.P2 / s.YT, s.nchunks, nm);
-    const int thr = s.YT * s.P1 / s.PPT;
-    const size_t sm = smem_sgs(s, sizeof(R) == 4, h->g.K1);
-    if (s.sx2) {
-        switch (s.P1) {
-            case 64: BLD_TRY((launch_sgs_x2_p<R, 64>(h, s, a, grid, thr, sm))); break;
-            case 96: BLD_TRY((launch_sgs_x2_p<R, 96>(h, s, a, grid, thr, sm))); break;
-            case 128: BLD_TRY((launch_sgs_x2_p<R, 128>(h, s, a, grid, thr, sm))); break;
-            case 144: BLD_TRY((launch_sgs_x2_p<R, 144>(h, s, a, grid, thr, sm))); break;
-            case 192: BLD_TRY((launch_sgs_x2_p<R, 192>(h, s, a, grid, thr, sm))); break;
-            case 256: BLD_TRY((launch_sgs_x2_p<R, 256>(h, s, a, grid, thr, sm))); break;
-            case 288: BLD_TRY((launch_sgs_x2_p<R, 288>(h, s, a, grid, thr, sm))); break;
-            default:
-                if constexpr (sizeof(R) == 4) {
-                    if (s.P1 == 384) { BLD_TRY((launch_sgs_x2_p<R, 384>(h, s, a, grid, thr, sm))); break; }
-                    if (s.P1 == 512) { BLD_TRY((launch_sgs_x2_p<R, 512>(h, s, a, grid, thr, sm))); break; }
-                    if (s.P1 == 768) { BLD_TRY((launch_sgs_x2_p<R, 768>(h, s, a, grid, thr, sm))); break; }
-                }
-                return fail(BLD_ERR_INVALID_CONFIG, "no two-pass SGS x kernel for P1=%d", s.P1);
-        }
-        CUDA_TRY(cudaGetLastError());
-        return BLD_OK;
-    }
-    if (s.xr) {
-        switch (s.xr) {
-            BLD_XR_CASES(k_sgs_x)
-            default: return fail(BLD_ERR_INVALID_CONFIG, "no warp x transform of radix %d", s.xr);
-        }
-    } else {
-        switch (s.PPT) {
-            case 1: k_sgs_x<R, 1, 0><<<grid, thr, sm, h->stream>>>(a); break;
-            case 2: k_sgs_x<R, 2, 0><<<grid, thr, sm, h->stream>>>(a); break;
-            case 3: k_sgs_x<R, 3, 0><<<grid, thr, sm, h->stream>>>(a); break;
-            default: k_sgs_x<R, 4, 0><<<grid, thr, sm, h->stream>>>(a); break;
-        }
-    }
-    CUDA_TRY(cudaGetLastError());
-    return BLD_OK;
-}
-
-template <typename R>
-int set_smem_limits_R() {
-    const int lim = 227 * 1024;   // the largest dynamic shared memory a B200 block may opt into
-    // large dynamic shared memory, and the largest shared-memory carveout so the
-    // per-SM block count is set by the kernel's real footprint
-#define BLD_SET(K)                                                                           \
-    do {                                                                                     \
-        CUDA_TRY(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)); \
-        CUDA_TRY(cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout,     \
-                                      cudaSharedmemCarveoutMaxShared));                      \
-    } while (0)
-    BLD_SET((k_inv_y<R, 0>));
-    BLD_SET((k_fwd_y<R, 0>));
-    BLD_SET((k_inv_y<R, 2>));
-    BLD_SET((k_fwd_y<R, 2>));
-    BLD_SET((k_inv_y<R, 3>));
-    BLD_SET((k_fwd_y<R, 3>));
-    BLD_SET((k_inv_y<R, 4>));
-    BLD_SET((k_fwd_y<R, 4>));
-    BLD_SET((k_inv_y<R, 6>));
-    BLD_SET((k_fwd_y<R, 6>));
-    BLD_SET((k_inv_y<R, 8>));
-    BLD_SET((k_fwd_y<R, 8>));
-    BLD_SET((k_inv_y<R, 9>));
-    BLD_SET((k_fwd_y<R, 9>));
-    BLD_SET((k_inv_y<R, 12>));
-    BLD_SET((k_fwd_y<R, 12>));
-    BLD_SET((k_inv_y<R, 16>));
-    BLD_SET((k_fwd_y<R, 16>));
-    if constexpr (sizeof(R) == 4) {
-        BLD_SET((k_inv_y<R, 24>));
-        BLD_SET((k_fwd_y<R, 24>));
-    }
-    BLD_SET((k_inv_y_all<R>));
-    BLD_SET((k_fwd_y_all<R>));
-#define BLD_SET_Y2(P)                                                                                  \
-    BLD_SET((k_inv_y2<R, y2_radix_a(P), y2_radix_b(P), y2_min_blocks_inv<R>(y2_radix_b(P) * BLD_Y2_NL)>)); \
-    BLD_SET((k_fwd_y2<R, y2_radix_a(P), y2_radix_b(P), y2_min_blocks<R>(y2_radix_b(P) * BLD_Y2_NL)>)); \
-    BLD_SET((k_fwd_y2<R, y2_radix_a(P), y2_radix_b(P), 3, 8, 4>));                                                                   \
-    BLD_SET((k_inv_y2<R, y2_radix_a(P), y2_radix_b(P), sizeof(R) == 8 ? 3 : 4, 8>));                                                \
-    if constexpr (sizeof(R) == 4)                                                                    \
-        BLD_SET((k_fwd_y2<R, y2_radix_a(P), y2_radix_b(P), y2_min_blocks<R>(y2_radix_b(P) * BLD_Y2_NL), BLD_Y2_NL, 2>));
-    BLD_SET_Y2(64)
-    BLD_SET_Y2(96)
-    BLD_SET_Y2(128)
-    BLD_SET_Y2(144)
-    BLD_SET_Y2(192)
-    BLD_SET_Y2(256)
-    BLD_SET_Y2(288)
-    if constexpr (sizeof(R) == 4) {
-        BLD_SET_Y2(384)
-        BLD_SET_Y2(512)
-        BLD_SET_Y2(768)
-    }
-#undef BLD_SET_Y2
-#define BLD_SET_Y3(P) BLD_SET((k_inv_y3<R, y2_radix_a(P), y2_radix_b(P)>));
-    BLD_SET_Y3(64)
-    BLD_SET_Y3(96)
-    BLD_SET_Y3(128)
-    BLD_SET_Y3(144)
-    BLD_SET_Y3(192)
-    BLD_SET_Y3(256)
-    BLD_SET_Y3(288)
-    if constexpr (sizeof(R) == 4) {
-        BLD_SET_Y3(384)
-        BLD_SET_Y3(512)
-        BLD_SET_Y3(768)
-    }
-#undef BLD_SET_Y3
-#define BLD_SET_X2(P)                                                   \
-    BLD_SET((k_adv_x2<R, y2_radix_a(P), y2_radix_b(P), 0>));            \
-    if constexpr (sizeof(R) == 8) {                                     \
-        BLD_SET((k_adv_x2<R, y2_radix_a(P), y2_radix_b(P), 2>));        \
-    }                                                                   \
-    if constexpr (sizeof(R) == 4 && P <= 384) {                         \
-        BLD_SET((k_adv_x2<R, y2_radix_a(P), y2_radix_b(P), 3>));        \
-    }
-    BLD_SET_X2(64)
-    BLD_SET_X2(96)
-    BLD_SET_X2(128)
-    BLD_SET_X2(144)
-    BLD_SET_X2(192)
-    BLD_SET_X2(256)
-    BLD_SET_X2(288)
-    if constexpr (sizeof(R) == 4) {
-        BLD_SET_X2(384)
-        BLD_SET_X2(512)
-        BLD_SET_X2(768)
-    }
-#undef BLD_SET_X2
-#define BLD_SET_SX2(P) BLD_SET((k_sgs_x<R, 1, 0, P>)); BLD_SET((k_sgs_x<R, 2, 0, P>));   \
-    if constexpr (P <= 288) BLD_SET((k_sgs_x2<R, y2_radix_a(P), y2_radix_b(P)>));          \
-    if constexpr (sizeof(R) == 4 && P <= 384) BLD_SET((k_sgs_x2<R, y2_radix_a(P), y2_radix_b(P), 1>));
-    BLD_SET_SX2(64)
-    BLD_SET_SX2(96)
-    BLD_SET_SX2(128)
-    BLD_SET_SX2(144)
-    BLD_SET_SX2(192)
-    BLD_SET_SX2(256)
-    BLD_SET_SX2(288)
-    if constexpr (sizeof(R) == 4) {
-        BLD_SET_SX2(384)
-        BLD_SET_SX2(512)
-        BLD_SET_SX2(768)
-        BLD_SET((k_sgs_x2<R, y2_radix_a(384), y2_radix_b(384)>));
-        BLD_SET((k_sgs_x2<R, y2_radix_a(512), y2_radix_b(512)>));
-        BLD_SET((k_sgs_x2<R, y2_radix_a(768), y2_radix_b(768)>));
-#define BLD_SET_SX2C(P) BLD_SET((k_sgs_x<R, 1, 0, P, 2>)); BLD_SET((k_sgs_x<R, 2, 0, P, 2>));
-        BLD_SET_SX2C(256)
-        BLD_SET_SX2C(288)
-        BLD_SET_SX2C(384)
-        BLD_SET_SX2C(512)
-        BLD_SET_SX2C(768)
-#undef BLD_SET_SX2C
-    }
-#undef BLD_SET_SX2
-    BLD_SET((k_adv_x<R, 1, 0>));
-    BLD_SET((k_adv_x<R, 2, 0>));
-    BLD_SET((k_adv_x<R, 3, 0>));
-    BLD_SET((k_adv_x<R, 4, 0>));
-    BLD_SET((k_sgs_x<R, 1, 0>));
-    BLD_SET((k_sgs_x<R, 2, 0>));
-    BLD_SET((k_sgs_x<R, 3, 0>));
-    BLD_SET((k_sgs_x<R, 4, 0>));
-#define BLD_SET_XR(r)                              \
-    BLD_SET((k_adv_x<R, xr_ppt(r), r>));           \
-    BLD_SET((k_sgs_x<R, xr_ppt(r), r>));
-    BLD_SET_XR(2)
-    BLD_SET_XR(3)
-    BLD_SET_XR(4)
-    BLD_SET_XR(6)
-    BLD_SET_XR(8)
-    BLD_SET_XR(9)
-    BLD_SET_XR(12)
-    BLD_SET_XR(16)
-    BLD_SET_XR(24)
-#undef BLD_SET_XR
-    BLD_SET((k_adv_xb<R, 2>));
-    BLD_SET((k_adv_xb<R, 3>));
-    BLD_SET((k_adv_xb<R, 4>));
-    BLD_SET((k_adv_xb<R, 6>));
-    BLD_SET((k_adv_xb<R, 8>));
-    BLD_SET((k_adv_xb<R, 9>));
-    BLD_SET((k_adv_xb<R, 12>));
-    BLD_SET((k_adv_xp<R, 2>));
-    BLD_SET((k_adv_xp<R, 3>));
-    BLD_SET((k_adv_xp<R, 4>));
-    BLD_SET((k_adv_xp<R, 6>));
-    BLD_SET((k_adv_xp<R, 8>));
-    BLD_SET((k_adv_xp<R, 9>));
-    BLD_SET((k_adv_xp<R, 12>));
-    if constexpr (sizeof(R) == 4) {
-        BLD_SET((k_adv_xb<R, 16>));
-        BLD_SET((k_adv_xb<R, 24>));
-        BLD_SET((k_adv_xp<R, 16>));
-        BLD_SET((k_adv_xp<R, 24>));
-    }
-    BLD_SET((k_adv_xw<R, 2>));
-    BLD_SET((k_adv_xw<R, 3>));
-    BLD_SET((k_adv_xw<R, 4>));
-    BLD_SET((k_adv_xw<R, 6>));
-    if constexpr (sizeof(R) == 4) {
-        BLD_SET((k_adv_xw<R, 8>));
-        BLD_SET((k_adv_xw<R, 9>));
-        BLD_SET((k_adv_xw<R, 12>));
-        BLD_SET((k_adv_xwc<R, 8, 3>));
-        BLD_SET((k_adv_xwc<R, 9, 3>));
-        BLD_SET((k_adv_xwc<R, 12, 3>));
-        BLD_SET((k_adv_xwc<R, 8, 4>));
-        BLD_SET((k_adv_xwc<R, 9, 4>));
-        BLD_SET((k_adv_xwc<R, 12, 4>));
-    }
-#undef BLD_SET
+        CUDA_TRY((h->fp32 ? bld_row::launch_sgs32 : bld_row::launch_sgs64)(a, s.nchunks, nm, h->stream));
     return BLD_OK;
 }
 
@@ -1186,6 +138,16 @@ int init_codelet_twiddles() {
         }
     CUDA_TRY(cudaMemcpyToSymbol(c_wtab64, h_wtab64, sizeof(h_wtab64)));
     CUDA_TRY(cudaMemcpyToSymbol(c_wtab32, h_wtab32, sizeof(h_wtab32)));
+    BLD_TRY(setup_y<double>());
+    BLD_TRY(setup_y<float>());
+    BLD_TRY(setup_adv<double>());
+    BLD_TRY(setup_adv<float>());
+    BLD_TRY(setup_sgs<double>());
+    BLD_TRY(setup_sgs<float>());
+    CUDA_TRY(bld_row::init_adv64());
+    CUDA_TRY(bld_row::init_adv32());
+    CUDA_TRY(bld_row::init_sgs64());
+    CUDA_TRY(bld_row::init_sgs32());
     done[dev] = true;
     return BLD_OK;
 }
@@ -1194,8 +156,6 @@ int set_smem_limits() {
     BLD_TRY(init_codelet_twiddles());
     static int done = 0;
     if (done) return BLD_OK;
-    BLD_TRY(set_smem_limits_R<double>());
-    BLD_TRY(set_smem_limits_R<float>());
     CUDA_TRY(cudaFuncSetAttribute(k_x_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(k_project_seg<8, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     // dynamic shared memory of k_project_tile: at most 200 KB (project_tile_ok)
@@ -1244,6 +204,14 @@ int enqueue_inv_y_R(bld_handle* h, int sp, const double2* state, int m0, int nm)
             ia.fld[i] = fl[i];
             ia.isI[i] = isI[i];
         }
+    } else if (s.xrow) {  // u, v, w, u_2, v_2, w_2: the x derivatives are taken by bld_row::k_sgs_x
+        const int op[6] = {T_DIRECT, T_DIRECT, T_DIRECT, T_D2, T_D2, T_D2};
+        ia.nterms = 6;
+        for (int i = 0; i < 6; ++i) {
+            ia.op[i] = op[i];
+            ia.fld[i] = i % 3;
+            ia.isI[i] = i % 3 == 2;
+        }
     } else {  // u, v, w, u_1, u_2, v_1, v_2, w_1, w_2 (src/processes/static_smagorinsky.jl:39-42)
         const int op[9] = {T_DIRECT, T_DIRECT, T_DIRECT, T_D1, T_D2, T_D1, T_D2, T_D1, T_D2};
         const int fl[9] = {0, 1, 2, 0, 0, 1, 1, 2, 2};
@@ -1288,10 +256,11 @@ int enqueue_x_R(bld_handle* h, int sp, int m0, int nm) {
     xa.p1_magic = fdiv_magic((unsigned)s.P1);
     xa.flag = h->flag;
     xa.active = h->mask_on ? h->active : nullptr;
+    xa.d1 = h->d1;
+    xa.wait_limit = h->wait_limit;
+    if (s.xrow) return launch_row(h, s, xa, nm);
     if (sp == 0) {
-        if (s.x2) return launch_adv_x2<R>(h, s, xa, nm);
-        if (s.xb) return launch_adv_xb<R>(h, s, xa, nm);
-        return s.xw ? launch_adv_xw<R>(h, s, xa, nm) : launch_adv_x<R>(h, s, xa, nm);
+        return launch_adv_family<R>(h, s, xa, nm);
     }
     return launch_sgs_x<R>(h, s, xa, nm);
 }
@@ -1318,6 +287,12 @@ int enqueue_fwd_y_R(bld_handle* h, int sp, bool first, bool last, const double2*
         for (int f = 0; f < 3; ++f) {
             fa.ncontrib[f] = 1;
             fa.c[f][0] = FwdContrib{f, 0};
+        }
+    } else if (s.xrow) {  // per component: d1 tau_i1 + d3 tau_i3 as one term, tau_i2
+        for (int f = 0; f < 3; ++f) {
+            fa.ncontrib[f] = 2;
+            fa.c[f][0] = FwdContrib{f, 0};
+            fa.c[f][1] = FwdContrib{3 + f, 2};
         }
     } else {  // rate order of add_rates! (src/physical_space.jl:191-204)
         fa.ncontrib[0] = 3;
@@ -1578,6 +553,7 @@ void copy_tuning(Space& dst, const Space& src) {
     dst.x2 = src.x2;
     dst.sx2 = src.sx2;
     dst.sxk = src.sxk;
+    dst.xrow = src.xrow;
     dst.inv = src.inv;
     dst.fwd = src.fwd;
 }
@@ -1669,8 +645,12 @@ int autotune_impl(bld_handle* h) {
         BLD_TRY(enqueue_inv_y(h, sp, h->u, 0, B));
         best = 1e30f;
         int byt = s.YT, bppt = s.PPT;
+        // the in-place kernels beat every other family where they are compiled (96 to 768
+        // points: 0.50 to 0.88 of the fastest other one's time), so only their z chunks are
+        // tuned there
+        const bool row = s.xrow != 0;
         for (auto c : x_candidates(h, s, sp == 0)) {
-            if ((sp == 0 && (only_warp || only_bw)) || only_lines) break;
+            if (row || (sp == 0 && (only_warp || only_bw)) || only_lines) break;
             s.YT = c.first;
             s.PPT = c.second;
             x_chunks(h, s);
@@ -1684,7 +664,7 @@ int autotune_impl(bld_handle* h) {
         // block x kernels with warp line transforms (YT = 1, 2)
         int bxr = 0;
         const int xrr = s.P1 % 32 ? 0 : s.P1 / 32;
-        if (xr_radix_ok(xrr) && !(sp == 0 && (only_warp || only_bw)) && !only_block && !xdisable_wlines()) {
+        if (!row && xr_radix_ok(xrr) && !(sp == 0 && (only_warp || only_bw)) && !only_block && !xdisable_wlines()) {
             for (int yt = 1; yt <= 2; ++yt) {
                 const size_t smx = (size_t)(s.P1 + 2 * (sp == 0 ? 3 : 5) * yt * (s.P1 + 32)) * csize(h->fp32);
                 if (s.P2 % yt || smx > 150 * 1024 || yt * s.P1 / xr_ppt(xrr) > 256) continue;
@@ -1704,7 +684,7 @@ int autotune_impl(bld_handle* h) {
         }
         // SGS: the block kernel with two-pass line transforms
         int bsx2 = 0;
-        if (sp == 1 && sx2_ok(h, s) && !only_block && !only_lines) {
+        if (!row && sp == 1 && sx2_ok(h, s) && !only_block && !only_lines) {
             float best2 = 1e30f;
             int yt2 = 1, ppt2 = 1, v2 = 1;
             for (int v = 1; v <= 4; ++v)
@@ -1743,9 +723,9 @@ int autotune_impl(bld_handle* h) {
         // its best z-chunk count (and, for the warp-per-row kernel, register
         // cap: more resident warps want more chunks)
         struct XPick {
-            int YT, PPT, xr, xw, xwmb, xb, zmult, x2, sx2, sxk;
+            int YT, PPT, xr, xw, xwmb, xb, zmult, x2, sx2, sxk, xrow;
         };
-        auto get_pick = [&]() { return XPick{s.YT, s.PPT, s.xr, s.xw, s.xwmb, s.xb, s.zmult, s.x2, s.sx2, s.sxk}; };
+        auto get_pick = [&]() { return XPick{s.YT, s.PPT, s.xr, s.xw, s.xwmb, s.xb, s.zmult, s.x2, s.sx2, s.sxk, s.xrow}; };
         auto set_pick = [&](const XPick& p) {
             s.YT = p.YT;
             s.PPT = p.PPT;
@@ -1757,6 +737,7 @@ int autotune_impl(bld_handle* h) {
             s.x2 = p.x2;
             s.sx2 = p.sx2;
             s.sxk = p.sxk;
+            s.xrow = p.xrow;
             x_chunks(h, s);
         };
         const char* mbe = getenv("BLD_XW_MINB");   // force one register cap (1, 3, 4)
@@ -1794,12 +775,12 @@ int autotune_impl(bld_handle* h) {
         const char* sxv = getenv("BLD_SGS_X2_VARIANT");
         const int sxv_only = sxv && sxv[0] ? atoi(sxv) : -1;
         for (int v = 0; v <= 1; ++v)
-            if (sp == 1 && sxk_ok(h, s, v) && (!sk || only_sxk) && (sxv_only < 0 || sxv_only == v))
+            if (!row && sp == 1 && sxk_ok(h, s, v) && (!sk || only_sxk) && (sxv_only < 0 || sxv_only == v))
                 BLD_TRY(tune_chunks(XPick{1, 1, 0, 0, 1, 0, 2, 0, 0, 1 + v}));
-        const bool warp_ok = sp == 0 && adv_warp_ok && !only_block && !only_bw && !only_lines && !only_x2;
+        const bool warp_ok = !row && sp == 0 && adv_warp_ok && !only_block && !only_bw && !only_lines && !only_x2;
         for (int wpb = 1; warp_ok && wpb <= 4; wpb *= 2) BLD_TRY(tune_chunks(XPick{1, 1, 0, wpb, 1, 0, 2, 0, 0, 0}));
         for (int xbk = 1; xbk <= 2; ++xbk) {
-            if (!(sp == 0 && adv_bw_ok && !only_block && !only_warp && !only_lines && !only_x2)) break;
+            if (row || !(sp == 0 && adv_bw_ok && !only_block && !only_warp && !only_lines && !only_x2)) break;
             if ((xbk == 1 && only_pipe) || (xbk == 2 && only_bw3)) continue;
             BLD_TRY(tune_chunks(XPick{1, 1, 0, 0, 1, xbk, 2, 0, 0, 0}));
         }
@@ -1807,8 +788,9 @@ int autotune_impl(bld_handle* h) {
         const char* x2v = getenv("BLD_X2_VARIANT");
         const int x2_only = x2v && x2v[0] ? atoi(x2v) : -1;
         for (int v = 0; v <= 3; ++v)
-            if (sp == 0 && x2_ok(h, s, v) && (only_x2 || !xk || x2_asked) && (x2_only < 0 || x2_only == v))
+            if (!row && sp == 0 && x2_ok(h, s, v) && (only_x2 || !xk || x2_asked) && (x2_only < 0 || x2_only == v))
                 BLD_TRY(tune_chunks(XPick{1, 1, 0, 0, 1, 0, 2, 1 + v, 0, 0}));
+        if (row) BLD_TRY(tune_chunks(XPick{1, 1, 0, 0, 1, 0, 2, 0, 0, 0, 1}));
         if (bx >= 1e30f) return fail(BLD_ERR_INVALID_CONFIG, "no x kernel could be timed");
         set_pick(bp);
         x_chunks(h, s);
@@ -1825,9 +807,9 @@ int autotune_impl(bld_handle* h) {
         s.fwd = bf;
         const char* v = getenv("BLD_VERBOSE");
         if (v && v[0] && v[0] != '0')
-            fprintf(stderr, "bld autotune %s P=%dx%d: inv all=%d NL=%d thr=%d wfft=%d tp=%d | x YT=%d PPT=%d xr=%d warps=%d bw=%d x2=%d sx2=%d sxk=%d chunks=%d | fwd all=%d NL=%d thr=%d wfft=%d tp=%d\n",
+            fprintf(stderr, "bld autotune %s P=%dx%d: inv all=%d NL=%d thr=%d wfft=%d tp=%d | x YT=%d PPT=%d xr=%d warps=%d bw=%d x2=%d sx2=%d sxk=%d row=%d chunks=%d | fwd all=%d NL=%d thr=%d wfft=%d tp=%d\n",
                     sp == 0 ? "advection" : "sgs", s.P1, s.P2, s.inv.all, s.inv.NL, s.inv.thr, s.inv.wfft, s.inv.tp, s.YT, s.PPT, s.xr, s.xw, (int)s.xb,
-                    s.x2, s.sx2, s.sxk, s.nchunks, s.fwd.all, s.fwd.NL, s.fwd.thr, s.fwd.wfft, s.fwd.tp);
+                    s.x2, s.sx2, s.sxk, s.xrow, s.nchunks, s.fwd.all, s.fwd.NL, s.fwd.thr, s.fwd.wfft, s.fwd.tp);
     }
     if (h->cfg.pressure && h->g.n3 <= 256) {
         float best = 1e30f, t = 0;
@@ -2233,8 +1215,9 @@ int setup_space(bld_handle* h, Space& s, int dealias, int e1, int e2, bool is_ad
     s.plan2 = make_plan(s.P2, h->fp32);
     BLD_TRY(twiddles(h, s.P1));
     BLD_TRY(twiddles(h, s.P2));
-    s.ntin = is_adv ? 6 : 9;
-    s.ntout = is_adv ? 3 : 8;
+    s.xrow = row_ok(h, s.P1, s.P2, is_adv) ? 1 : 0;
+    s.ntin = is_adv || s.xrow ? 6 : 9;
+    s.ntout = is_adv ? 3 : (s.xrow ? 6 : 8);
     s.fsets = is_adv ? 1 : 2;
     tile_space(h, s, is_adv);
     if (!s.PPT) return fail(BLD_ERR_INVALID_CONFIG, "no thread tiling for physical size %d", s.P1);
@@ -2374,6 +1357,10 @@ int32_t bld_create(const bld_config* cfg, bld_handle** out) {
     g.F = g.K1 * g.K2;
     g.mstride = (long long)(3 * g.n3 - 1) * g.F;
     const int n3 = g.n3, K1 = g.K1, K2 = g.K2, B = h->B;
+    if (cudaGetSymbolAddress((void**)&h->wait_limit, g_bld_wait_limit) != cudaSuccess) {
+        delete h;
+        return fail(BLD_ERR_CUDA, "cudaGetSymbolAddress failed");
+    }
     auto bail = [&](int code) {
         free_handle(h);
         return code;
@@ -2940,7 +1927,11 @@ int32_t bld_set_wait_limit(int32_t device, int64_t cycles) {
     CUDA_TRY(cudaGetDevice(&prev));
     CUDA_TRY(cudaSetDevice(device));
     const long long v = cycles < 0 ? BLD_WAIT_CYCLES : (long long)cycles;
-    const cudaError_t e = cudaMemcpyToSymbol(g_bld_wait_limit, &v, sizeof(v));
+    cudaError_t e = cudaMemcpyToSymbol(g_bld_wait_limit, &v, sizeof(v));
+    // every translation unit with bounded waits has its own copy
+    for (auto set : {wait_limit_y<double>, wait_limit_y<float>, wait_limit_adv<double>, wait_limit_adv<float>,
+                     wait_limit_sgs<double>, wait_limit_sgs<float>})
+        if (e == cudaSuccess) e = set(v);
     cudaSetDevice(prev);
     CUDA_TRY(e);
     return BLD_OK;
@@ -2990,7 +1981,10 @@ int32_t bld_describe(bld_handle* h, char* buf, size_t len) {
         char tmp[768];
         const char* xk = sp == 0 ? "k_adv_x" : "k_sgs_x";
         char xname[96];
-        if (sp == 0 && s.x2)
+        if (s.xrow)
+            snprintf(xname, sizeof xname, "%s<%s, %d, %d>", sp == 0 ? "k_adv_row" : "k_sgs_x", R, row_shape(h, s).A,
+                     row_shape(h, s).B);
+        else if (sp == 0 && s.x2)
             snprintf(xname, sizeof xname, "k_adv_x2<%s, %d, %d%s>", R, y2_radix_a(s.P1), y2_radix_b(s.P1),
                      s.x2 == 3 ? ", wide" : (s.x2 == 4 ? ", 2 rows" : ""));
         else if (sp == 0 && s.xb)
@@ -3020,7 +2014,7 @@ int32_t bld_describe(bld_handle* h, char* buf, size_t len) {
                  "%s\"%s\": {\"P\": [%d, %d], \"inv_y\": \"%s\", \"x\": \"%s\", \"fwd_y\": \"%s\", "
                  "\"inv_NL\": %d, \"fwd_NL\": %d, \"x_rows\": %d, \"x_chunks\": %d}",
                  out.size() > 1 ? ", " : "", sp == 0 ? "advection" : "sgs", s.P1, s.P2, iname, xname, fname, s.inv.NL,
-                 s.fwd.NL, s.xb ? 1 : (s.xw ? s.xw : s.YT), s.nchunks);
+                 s.fwd.NL, s.xrow ? row_shape(h, s).NR : s.xb ? 1 : (s.xw ? s.xw : s.YT), s.nchunks);
         out += tmp;
     }
     char tmp[160];

@@ -21,6 +21,7 @@
 #include "bld_dft.cuh"
 #include "bld_warpfft.cuh"
 #include "bld_tma.cuh"
+#include "bld_xargs.cuh"
 
 #define BLD_MAXT 10
 #define BLD_MAXC 4
@@ -32,17 +33,6 @@ __host__ __device__ constexpr int y2_radix_a(int P) {
          : P == 384 ? 16 : P == 512 ? 16 : P == 768 ? 24 : 0;
 }
 __host__ __device__ constexpr int y2_radix_b(int P) { return y2_radix_a(P) ? P / y2_radix_a(P) : 0; }
-
-struct Geo {
-    int K1, K2, k1max, k2max, n3, F;  // F = K1*K2 modes per layer
-    long long mstride;                // complex values per member state (3*n3-1)*F
-};
-
-__host__ __device__ __forceinline__ long long fld_off(const Geo& g, int f) { return (long long)f * g.n3 * g.F; }
-
-// inactive ensemble slots (serving) skip their blocks; uniform per block
-#define BLD_SKIP_INACTIVE(a, m) \
-    if ((a).active && !(a).active[m]) return
 
 // Copies n table entries from global to shared memory with up to 8 loads in
 // flight per thread (a load-then-store loop would wait one DRAM latency per entry).
@@ -373,55 +363,6 @@ __global__ void __launch_bounds__(384) k_inv_y_all(InvYArgs a) {
 }
 
 // ----------------------------------------------------------- physical x kernels
-struct XArgs {
-    Geo g;
-    int P1, P2, YT, zchunk;
-    int m0;
-    const int* active;
-    const void* min;
-    void* mout;
-    long long min_mstride, mout_mstride;  // elements per member
-    FftPlan plan;
-    const void* tw;
-    // SGS only
-    const double* alpha_c;   // [n3]
-    const double* alpha_i;   // [n3-1]
-    const double* lc;        // [members][n3]   Smagorinsky length^2 at C nodes
-    const double* li;        // [members][n3-1] ... at I nodes
-    const double* wall;      // [members][4]: strain factor lo, hi; stress factor lo, hi
-    int dyn_lo, dyn_hi;      // rough wall (dynamic wall-model values) below / above
-    double w_lo, w_hi;       // Dirichlet values of vel3
-    // two-pass SGS kernel: the input rows of layer j + 1 are copied into shared
-    // memory by 1-d TMA bulk copies while layer j is processed (needs YT K1
-    // elements to fill whole 16-byte units); a timed-out wait sets flag[m]
-    int staged;
-    int* flag;
-    // ceil(2^32 / K1) and ceil(2^32 / P1) (0 for a divisor of 1): fdiv
-    unsigned k1_magic, p1_magic;
-};
-
-// n / d for 0 <= n < 2^16 and 1 <= d < 2^16 by one multiply-high with
-// magic = ceil(2^32 / d) (0 for d = 1): with n = q d + r, n magic / 2^32 exceeds
-// n / d by less than 2^-16 <= 1 / d, so its floor is q.  Replaces runtime integer
-// divisions (tens of instructions each) in the index arithmetic of the x kernels.
-__host__ __device__ __forceinline__ int fdiv(int n, unsigned magic) {
-#ifdef __CUDA_ARCH__
-    return magic ? (int)__umulhi((unsigned)n, magic) : n;
-#else
-    return magic ? (int)(((unsigned long long)(unsigned)n * magic) >> 32) : n;
-#endif
-}
-inline unsigned fdiv_magic(unsigned d) { return d <= 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
-
-template <typename C>
-__device__ __forceinline__ const C* mrow(const C* M, const XArgs& a, int t, int z, int y) {
-    return M + ((long long)(t * a.g.n3 + z) * a.P2 + y) * a.g.K1;
-}
-template <typename C>
-__device__ __forceinline__ C* mrow_w(C* M, const XArgs& a, int t, int z, int y) {
-    return M + ((long long)(t * a.g.n3 + z) * a.P2 + y) * a.g.K1;
-}
-
 // Build packed line Z[k] = A[k] + i B[k] (Hermitian-extended, DC imaginary parts
 // dropped as in FFTW's c2r) from mixed rows A (term ta) and B (term tb).
 template <typename R>
@@ -1590,7 +1531,7 @@ __global__ void __launch_bounds__(384) k_fwd_y_all(FwdYArgs a) {
 }
 
 // Linear terms only (no physical-domain process): grid (ceil(F/256), n3, 3*members)
-__global__ void __launch_bounds__(256) k_linear(FwdYArgs a) {
+static __global__ void __launch_bounds__(256) k_linear(FwdYArgs a) {
     const Geo& g = a.g;
     const int f = blockIdx.z % 3, m = a.m0 + blockIdx.z / 3;
     BLD_SKIP_INACTIVE(a, m);
@@ -1710,7 +1651,7 @@ __device__ __forceinline__ double2 stage_value_k(const ProjArgs& a, long long id
 // One thread per (k1, k2) column: stage update, divergence (div!, src/processes/pressure.jl:368-378),
 // forward/backward Thomas (:106-165), gradient (add_gradient!, :405-426), then ConstantMean
 // (src/processes/sources.jl:71-77) on the (0,0) column.  grid (ceil(F/128), members)
-__global__ void __launch_bounds__(128) k_project(ProjArgs a) {
+static __global__ void __launch_bounds__(128) k_project(ProjArgs a) {
     const Geo& g = a.g;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int m = a.m0 + blockIdx.y;
@@ -2215,7 +2156,7 @@ struct XPlainArgs {
 };
 
 // r2c along x of two physical rows per block -> mixed rows; grid ceil(nz*P2/2)
-__global__ void __launch_bounds__(256) k_x_r2c(XPlainArgs a) {
+static __global__ void __launch_bounds__(256) k_x_r2c(XPlainArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* tw = reinterpret_cast<double2*>(smem_raw);
     double2* b0 = tw + a.P1;
@@ -2239,7 +2180,7 @@ __global__ void __launch_bounds__(256) k_x_r2c(XPlainArgs a) {
 }
 
 // c2r along x of two mixed rows per block -> physical rows; grid ceil(nz*P2/2)
-__global__ void __launch_bounds__(256) k_x_c2r(XPlainArgs a) {
+static __global__ void __launch_bounds__(256) k_x_c2r(XPlainArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* tw = reinterpret_cast<double2*>(smem_raw);
     double2* b0 = tw + a.P1;
@@ -2264,7 +2205,7 @@ __global__ void __launch_bounds__(256) k_x_c2r(XPlainArgs a) {
 // Half-grid-point shift of one field in the frequency domain (shift!/unshift!,
 // src/physical_space.jl:321-336): q(k1, k2) *= exp(sign i pi (k1/P1 + k2/P2)) for
 // the default physical size (P1, P2).  grid (ceil(F/256), nz), dst may equal src.
-__global__ void __launch_bounds__(256) k_half_shift(double2* dst, const double2* __restrict__ src, Geo g, int P1, int P2,
+static __global__ void __launch_bounds__(256) k_half_shift(double2* dst, const double2* __restrict__ src, Geo g, int P1, int P2,
                                                      double sign) {
     const int mo = blockIdx.x * blockDim.x + threadIdx.x;
     if (mo >= g.F) return;
@@ -2284,7 +2225,7 @@ __global__ void __launch_bounds__(256) k_half_shift(double2* dst, const double2*
 // which stay zero as in log_state!); acc += w (prev + sample) adds one trapezoid,
 // and prev takes the new sample.  w = 0 only records the sample.
 // grid (members), block 128.
-__global__ void __launch_bounds__(128) k_profile_sample(Geo g, const double2* __restrict__ u, double* acc, double* prev,
+static __global__ void __launch_bounds__(128) k_profile_sample(Geo g, const double2* __restrict__ u, double* acc, double* prev,
                                                          double w, int m0, const int* active) {
     const int m = m0 + blockIdx.x;
     if (active && !active[m]) return;
@@ -2314,7 +2255,7 @@ __global__ void __launch_bounds__(128) k_profile_sample(Geo g, const double2* __
 // stored); the physical grids that sample a field band-limited to |k| <= kmax
 // hold at least 2 kmax + 1 points, so both are exact (ProgressMonitor,
 // src/logging.jl:246-266).  grid (n3, 3), block 256; out[(f n3 + z) 2 + {0,1}].
-__global__ void __launch_bounds__(256) k_progress_modes(Geo g, const double2* __restrict__ S, double* out) {
+static __global__ void __launch_bounds__(256) k_progress_modes(Geo g, const double2* __restrict__ S, double* out) {
     const int z = blockIdx.x, f = blockIdx.y;
     if (f == 2 && z >= g.n3 - 1) return;
     const double2* L = S + fld_off(g, f) + (long long)z * g.F;
@@ -2338,7 +2279,7 @@ __global__ void __launch_bounds__(256) k_progress_modes(Geo g, const double2* __
 }
 
 // max |v| over each of `nz` physical layers of n points; grid nz, block 256
-__global__ void __launch_bounds__(256) k_layer_absmax(const double* __restrict__ v, long long n, double* out) {
+static __global__ void __launch_bounds__(256) k_layer_absmax(const double* __restrict__ v, long long n, double* out) {
     const double* L = v + (long long)blockIdx.x * n;
     double mx = 0.0;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, fabs(L[i]));
@@ -2356,7 +2297,7 @@ __global__ void __launch_bounds__(256) k_layer_absmax(const double* __restrict__
 // over one physical layer of n points of u_1 (pu) and u_2 (pv)
 // (stress_bc, src/processes/static_smagorinsky.jl:195-200; hmean,
 // src/logging.jl:411-413).  One block of 256; out[0] tau13, out[1] tau23.
-__global__ void __launch_bounds__(256) k_wall_stress_mean(const double* __restrict__ pu, const double* __restrict__ pv,
+static __global__ void __launch_bounds__(256) k_wall_stress_mean(const double* __restrict__ pu, const double* __restrict__ pv,
                                                           long long n, double factor, double* out) {
     double s1 = 0.0, s2 = 0.0;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) {
@@ -2409,7 +2350,7 @@ struct InitTables {
 // 2 u - 1 with u = (splitmix64(key + 2 i) >> 11) 2^-53) or standard normal
 // (distribution 1: Box-Muller, sqrt(-2 log(1 - u)) cos(2 pi u') with u' from
 // key + 2 i + 1).  Grid-stride loop.
-__global__ void __launch_bounds__(256) k_init_random(double* __restrict__ pd, int plane, int nz, InitTables t,
+static __global__ void __launch_bounds__(256) k_init_random(double* __restrict__ pd, int plane, int nz, InitTables t,
                                                      int distribution, uint64_t key) {
     const long long n = (long long)nz * plane;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {

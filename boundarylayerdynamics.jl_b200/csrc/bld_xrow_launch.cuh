@@ -1,0 +1,79 @@
+// Launchers of the in-place x kernels; each translation unit instantiates one of them.
+#pragma once
+
+#include <atomic>
+
+#include "bld_xrow.h"
+#include "bld_xrows.cuh"
+
+namespace bld_row {
+
+inline cudaError_t init_tables() {
+    cudaError_t e = cudaMemcpyToSymbol(c_wtab64, h_wtab64, sizeof(h_wtab64));
+    return e == cudaSuccess ? cudaMemcpyToSymbol(c_wtab32, h_wtab32, sizeof(h_wtab32)) : e;
+}
+
+// opts `kernel` in to `smem` bytes and the largest shared-memory carveout on the current
+// device, the first time and whenever more bytes are asked for
+template <typename K>
+cudaError_t opt_in(K kernel, int smem, std::atomic<int> (&done)[64]) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 64 && done[dev].load() >= smem) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess && dev < 64) done[dev].store(smem);
+    return e;
+}
+
+template <typename R, int P>
+cudaError_t launch_adv_p(const XArgs& a, int nchunks, int nm, cudaStream_t st) {
+    constexpr Shape s = adv_shape(P, sizeof(R) == 4);
+    if constexpr (s.A > 0) {
+        static std::atomic<int> done[64];
+        const auto k = k_adv_row<R, s.A, s.B, s.NR, s.T, s.MINB, s.sepf>;
+        const int sm = ar_smem(s.A, s.B, a.g.K1, (int)sizeof(cplx<R>), s.NR, s.sepf);
+        if (const cudaError_t e = opt_in(k, sm, done); e != cudaSuccess) return e;
+        k<<<dim3(a.P2 / s.NR, nchunks, nm), s.T, sm, st>>>(a);
+        return cudaGetLastError();
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <typename R, int P>
+cudaError_t launch_sgs_p(const XArgs& a, int nchunks, int nm, cudaStream_t st) {
+    constexpr Shape s = sgs_shape(P, sizeof(R) == 4);
+    if constexpr (s.A > 0) {
+        static std::atomic<int> done[64];
+        const auto k = k_sgs_x<R, s.A, s.B, s.NR, s.T, s.MINB, s.sepf>;
+        const int sm = sr_smem(s.A, s.B, a.g.K1, (int)sizeof(cplx<R>), s.NR, s.sepf);
+        if (const cudaError_t e = opt_in(k, sm, done); e != cudaSuccess) return e;
+        k<<<dim3(a.P2 / s.NR, nchunks, nm), s.T, sm, st>>>(a);
+        return cudaGetLastError();
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <typename R>
+cudaError_t launch_adv(const XArgs& a, int nchunks, int nm, cudaStream_t st) {
+    switch (a.P1) {
+#define X(N) case N: return launch_adv_p<R, N>(a, nchunks, nm, st);
+        BLD_ROW_ADV_SIZES(X)
+#undef X
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+template <typename R>
+cudaError_t launch_sgs(const XArgs& a, int nchunks, int nm, cudaStream_t st) {
+    switch (a.P1) {
+#define X(N) case N: return launch_sgs_p<R, N>(a, nchunks, nm, st);
+        BLD_ROW_SGS_SIZES(X)
+#undef X
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace bld_row
