@@ -212,6 +212,8 @@ struct bld_handle {
     std::map<std::pair<int, double>, cudaGraph_t> graph_src;   // kept for ensemble parent graphs
     std::map<std::vector<const void*>, cudaGraphExec_t> ens_graphs;  // parent graphs led by this handle
     size_t bytes = 0;
+    cudaStream_t side = nullptr;   // second branch of the right-hand side (with both physical spaces)
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 };
 
 namespace bld {
