@@ -10,6 +10,7 @@
 
 #include "bld_engine.h"
 #include "bld_project_tile.cuh"
+#include "bld_yline.h"
 
 double2 h_wtab64[BLD_WTAB_SIZE];
 float2 h_wtab32[BLD_WTAB_SIZE];
@@ -113,6 +114,14 @@ bool row_ok(const bld_handle* h, int P1, int P2, bool is_adv) {
     if (!(is_adv ? bld_row::adv_compiled(P1, h->fp32) : bld_row::sgs_compiled(P1, h->fp32)) || P2 % r.NR) return false;
     return is_adv ? P1 % 3 != 0 || 3 * h->g.k1max < P1 : P1 == 2 * h->g.k1max + 2;
 }
+// The line y passes: compiled for the sizes of bld_yline.h; the 3/2 rule's empty middle
+// third where P2 is a multiple of 3 (advection), the default grid with the six mixed terms
+// of the in-place kernel (Smagorinsky).  BLD_Y_KERNEL asks for another family.
+bool yline_ok(const bld_handle* h, int P2, bool is_adv, bool xrow) {
+    const char* e = getenv("BLD_Y_KERNEL");
+    if ((e && e[0] && strcmp(e, "lines")) || !bld_yl::compiled(P2, h->fp32, !is_adv)) return false;
+    return is_adv ? P2 % 3 != 0 || 3 * h->g.k2max < P2 : xrow && P2 == 2 * h->g.k2max + 2;
+}
 int launch_row(bld_handle* h, const Space& s, const XArgs& a, int nm) {
     if (&s == &h->adv)
         CUDA_TRY((h->fp32 ? bld_row::launch_adv32 : bld_row::launch_adv64)(a, s.nchunks, nm, h->stream));
@@ -144,6 +153,11 @@ int init_codelet_twiddles() {
     BLD_TRY(setup_adv<float>());
     BLD_TRY(setup_sgs<double>());
     BLD_TRY(setup_sgs<float>());
+#define X(U)                             \
+    CUDA_TRY(bld_yl::init_inv_##U());    \
+    CUDA_TRY(bld_yl::init_fwd_##U());
+    BLD_YL_UNITS(X)
+#undef X
     CUDA_TRY(bld_row::init_adv64());
     CUDA_TRY(bld_row::init_adv32());
     CUDA_TRY(bld_row::init_sgs64());
@@ -222,6 +236,11 @@ int enqueue_inv_y_R(bld_handle* h, int sp, const double2* state, int m0, int nm)
             ia.fld[i] = fl[i];
             ia.isI[i] = isI[i];
         }
+    }
+    if (s.yl) {
+        if (sp == 0) CUDA_TRY((sizeof(R) == 4 ? bld_yl::launch_inv_adv32 : bld_yl::launch_inv_adv64)(ia, nm, h->stream));
+        else CUDA_TRY((sizeof(R) == 4 ? bld_yl::launch_inv_sgs32 : bld_yl::launch_inv_sgs64)(ia, nm, h->stream));
+        return BLD_OK;
     }
     return launch_inv_y<R>(h, s, ia, nm);
 }
@@ -325,7 +344,7 @@ int enqueue_fwd_y_R(bld_handle* h, int sp, bool first, bool last, const double2*
     fa.plan = s.plan2;
     fa.tw = twp(h, s.P2, sizeof(R) == 4);
     if (sf) {
-        if (s.fwd.all) return fail(BLD_ERR_INVALID_CONFIG, "stage fusion needs the per-term forward y kernel");
+        if (s.fwd.all && !s.yl) return fail(BLD_ERR_INVALID_CONFIG, "stage fusion needs the per-term forward y kernel");
         fa.fuse = 1;
         fa.su = sf->su;
         fa.sout = sf->sout;
@@ -333,6 +352,11 @@ int enqueue_fwd_y_R(bld_handle* h, int sp, bool first, bool last, const double2*
         fa.st_ct = sf->ct;
         fa.st_cd = sf->cd;
         fa.st_inv = 1.0 / sf->div;
+    }
+    if (s.yl) {
+        if (sp == 0) CUDA_TRY((sizeof(R) == 4 ? bld_yl::launch_fwd_adv32 : bld_yl::launch_fwd_adv64)(fa, nm, h->stream));
+        else CUDA_TRY((sizeof(R) == 4 ? bld_yl::launch_fwd_sgs32 : bld_yl::launch_fwd_sgs64)(fa, nm, h->stream));
+        return BLD_OK;
     }
     return launch_fwd_y<R>(h, s, fa, nm);
 }
@@ -554,6 +578,7 @@ void copy_tuning(Space& dst, const Space& src) {
     dst.sx2 = src.sx2;
     dst.sxk = src.sxk;
     dst.xrow = src.xrow;
+    dst.yl = src.yl;
     dst.inv = src.inv;
     dst.fwd = src.fwd;
 }
@@ -634,6 +659,7 @@ int autotune_impl(bld_handle* h) {
         float best = 1e30f, t = 0;
         YCfg bi = s.inv;
         for (const YCfg& c : y_candidates(h, s, 1, s.ntin, true)) {
+            if (s.yl) break;   // the line passes are the fastest where they are compiled
             s.inv = c;
             BLD_TRY(time_launches(h, [&] { return enqueue_inv_y(h, sp, h->u, 0, B); }, 3, &t));
             if (t < best) {
@@ -797,6 +823,7 @@ int autotune_impl(bld_handle* h) {
         best = 1e30f;
         YCfg bf = s.fwd;
         for (const YCfg& c : y_candidates(h, s, s.fsets, 3 * s.fsets, false)) {
+            if (s.yl) break;
             s.fwd = c;
             BLD_TRY(time_launches(h, [&] { return enqueue_fwd_y(h, sp, true, false, h->u, h->io2, 0, B); }, 3, &t));
             if (t < best) {
@@ -938,7 +965,7 @@ bool stage_fusable(const bld_handle* h) {
     if (e && e[0] && e[0] != '0') return false;
     if (!h->adv.on && !h->sgs.on) return false;
     const Space& last = h->sgs.on ? h->sgs : h->adv;
-    return !last.fwd.all;
+    return last.yl || !last.fwd.all;
 }
 
 // steps of one call may be chained (BLD_NO_STEP_CHAIN=1 keeps every step whole)
@@ -1244,6 +1271,7 @@ int setup_space(bld_handle* h, Space& s, int dealias, int e1, int e2, bool is_ad
     BLD_TRY(twiddles(h, s.P1));
     BLD_TRY(twiddles(h, s.P2));
     s.xrow = row_ok(h, s.P1, s.P2, is_adv) ? 1 : 0;
+    s.yl = yline_ok(h, s.P2, is_adv, s.xrow != 0) ? 1 : 0;
     s.ntin = is_adv || s.xrow ? 6 : 9;
     s.ntout = is_adv ? 3 : (s.xrow ? 6 : 8);
     s.fsets = is_adv ? 1 : 2;
@@ -2037,20 +2065,24 @@ int32_t bld_describe(bld_handle* h, char* buf, size_t len) {
         else
             snprintf(xname, sizeof xname, "%s<%s, %d, %d>", xk, R, s.PPT, s.xr);
         char iname[64], fname[64];
-        if (s.inv.tp == 2) snprintf(iname, sizeof iname, "k_inv_y3<%s, %d, %d>", R, y2_radix_a(s.P2), y2_radix_b(s.P2));
+        const bld_yl::Shape yi = s.yl ? bld_yl::inv_shape(s.P2, h->fp32, sp == 1) : bld_yl::Shape{};
+        const bld_yl::Shape yf = s.yl ? bld_yl::fwd_shape(s.P2, h->fp32, sp == 1) : bld_yl::Shape{};
+        if (s.yl) snprintf(iname, sizeof iname, "k_inv_yl<%s, %d, %d, %d lines>", R, yi.A, yi.B, yi.NL);
+        else if (s.inv.tp == 2) snprintf(iname, sizeof iname, "k_inv_y3<%s, %d, %d>", R, y2_radix_a(s.P2), y2_radix_b(s.P2));
         else if (s.inv.tp) snprintf(iname, sizeof iname, "k_inv_y2<%s, %d, %d%s>", R, y2_radix_a(s.P2), y2_radix_b(s.P2),
                                     s.inv.tp == 3 ? ", 8 lines" : "");
         else if (s.inv.all) snprintf(iname, sizeof iname, "k_inv_y_all<%s>", R);
         else snprintf(iname, sizeof iname, "k_inv_y<%s, %d>", R, s.inv.wfft);
-        if (s.fwd.tp) snprintf(fname, sizeof fname, "k_fwd_y2<%s, %d, %d%s>", R, y2_radix_a(s.P2), y2_radix_b(s.P2),
+        if (s.yl) snprintf(fname, sizeof fname, "k_fwd_yl<%s, %d, %d, %d lines>", R, yf.A, yf.B, yf.NL);
+        else if (s.fwd.tp) snprintf(fname, sizeof fname, "k_fwd_y2<%s, %d, %d%s>", R, y2_radix_a(s.P2), y2_radix_b(s.P2),
                                s.fwd.tp == 3 ? ", 8 lines" : (s.fwd.tp == 4 ? ", 2 outputs" : ""));
         else if (s.fwd.all) snprintf(fname, sizeof fname, "k_fwd_y_all<%s>", R);
         else snprintf(fname, sizeof fname, "k_fwd_y<%s, %d>", R, s.fwd.wfft);
         snprintf(tmp, sizeof tmp,
                  "%s\"%s\": {\"P\": [%d, %d], \"inv_y\": \"%s\", \"x\": \"%s\", \"fwd_y\": \"%s\", "
                  "\"inv_NL\": %d, \"fwd_NL\": %d, \"x_rows\": %d, \"x_chunks\": %d}",
-                 out.size() > 1 ? ", " : "", sp == 0 ? "advection" : "sgs", s.P1, s.P2, iname, xname, fname, s.inv.NL,
-                 s.fwd.NL, s.xrow ? row_shape(h, s).NR : s.xb ? 1 : (s.xw ? s.xw : s.YT), s.nchunks);
+                 out.size() > 1 ? ", " : "", sp == 0 ? "advection" : "sgs", s.P1, s.P2, iname, xname, fname, s.yl ? yi.NL : s.inv.NL,
+                 s.yl ? yf.NL : s.fwd.NL, s.xrow ? row_shape(h, s).NR : s.xb ? 1 : (s.xw ? s.xw : s.YT), s.nchunks);
         out += tmp;
     }
     char tmp[160];

@@ -149,6 +149,7 @@ struct Space {
     int xr = 0;                                     // block x kernels: warp-transform radix (P1 = 32 xr), 0 = Stockham
     int fsets = 1;                                  // forward line sets (2 when a D2 contribution exists)
     YCfg inv, fwd;                                  // y-pass variants (chosen by the autotuner)
+    int yl = 0;                                     // 1: the line y passes k_inv_yl / k_fwd_yl (bld_ylines.cuh) instead
 };
 
 }  // namespace bld

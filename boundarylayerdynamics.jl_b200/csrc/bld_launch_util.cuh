@@ -1,0 +1,34 @@
+// Helpers of the translation units that hold kernels: codelet tables and opt-in to large
+// dynamic shared memory.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <atomic>
+
+#include "bld_dft.cuh"
+
+namespace bld_util {
+
+// copies the codelet twiddles to this translation unit's tables on the current device
+inline cudaError_t init_tables() {
+    cudaError_t e = cudaMemcpyToSymbol(c_wtab64, h_wtab64, sizeof(h_wtab64));
+    return e == cudaSuccess ? cudaMemcpyToSymbol(c_wtab32, h_wtab32, sizeof(h_wtab32)) : e;
+}
+
+// opts `kernel` in to `smem` bytes and the largest shared-memory carveout on the current
+// device, the first time and whenever more bytes are asked for
+template <typename K>
+cudaError_t opt_in(K kernel, int smem, std::atomic<int> (&done)[64]) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 64 && done[dev].load() >= smem) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess && dev < 64) done[dev].store(smem);
+    return e;
+}
+
+}  // namespace bld_util

@@ -1,32 +1,14 @@
 // Launchers of the in-place x kernels; each translation unit instantiates one of them.
 #pragma once
 
-#include <atomic>
-
+#include "bld_launch_util.cuh"
 #include "bld_xrow.h"
 #include "bld_xrows.cuh"
 
 namespace bld_row {
 
-inline cudaError_t init_tables() {
-    cudaError_t e = cudaMemcpyToSymbol(c_wtab64, h_wtab64, sizeof(h_wtab64));
-    return e == cudaSuccess ? cudaMemcpyToSymbol(c_wtab32, h_wtab32, sizeof(h_wtab32)) : e;
-}
-
-// opts `kernel` in to `smem` bytes and the largest shared-memory carveout on the current
-// device, the first time and whenever more bytes are asked for
-template <typename K>
-cudaError_t opt_in(K kernel, int smem, std::atomic<int> (&done)[64]) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 64 && done[dev].load() >= smem) return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess && dev < 64) done[dev].store(smem);
-    return e;
-}
+using bld_util::init_tables;
+using bld_util::opt_in;
 
 template <typename R, int P>
 cudaError_t launch_adv_p(const XArgs& a, int nchunks, int nm, cudaStream_t st) {
