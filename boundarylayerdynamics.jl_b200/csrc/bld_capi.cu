@@ -111,7 +111,7 @@ bool row_ok(const bld_handle* h, int P1, int P2, bool is_adv) {
         if (e && e[0] && strcmp(e, "inplace")) return false;
     }
     const bld_row::Shape r = is_adv ? bld_row::adv_shape(P1, h->fp32) : bld_row::sgs_shape(P1, h->fp32);
-    if (!(is_adv ? bld_row::adv_compiled(P1, h->fp32) : bld_row::sgs_compiled(P1, h->fp32)) || P2 % r.NR) return false;
+    if (!(is_adv ? bld_row::adv_compiled(P1, h->fp32) : bld_row::sgs_compiled(P1, h->fp32)) || P2 % (is_adv ? 2 : r.NR)) return false;
     return is_adv ? P1 % 3 != 0 || 3 * h->g.k1max < P1 : P1 == 2 * h->g.k1max + 2;
 }
 // The line y passes: compiled for the sizes of bld_yline.h; the 3/2 rule's empty middle

@@ -37,11 +37,13 @@ constexpr void factor(Shape& s, int P, bool fp32, int multiple) {
     }
 }
 
-// Advection.  Threads: one per task of the wider inverse pass, rounded down where that
-// leaves few idle (measured: 288 points, double 96 / 128 / 192 threads 0.195 / 0.181 /
-// 0.237 ms at 192^2 x 96, single 0.099 / 0.105 / 0.114 ms).  Blocks per SM: the most
-// whose register cap does not spill.  384 points and above in double precision share
-// the line buffer between both directions, for three blocks per SM (0.234 against
+// Advection.  Threads: about one per task of the inverse passes, so that few idle in the
+// others (288 points, double: 96 / 128 / 192 threads 0.195 / 0.181 / 0.237 ms at
+// 192^2 x 96, single 0.099 / 0.105 / 0.114 ms).  Four rows per block up to 216 points in
+// single precision (two against four rows: 96 points 103 / 89 us at 64^2 x 768, 144 points
+// 136 / 117 us at 96^2 x 512), two elsewhere (registers, shared memory).  Blocks per SM:
+// the most whose register cap does not spill.  384 points and above in double precision
+// share the line buffer between both directions, for three blocks per SM (0.234 against
 // 0.244 ms with two at 256^2 x 64).
 constexpr Shape adv_shape(int P, bool fp32) {
     Shape s;
@@ -55,9 +57,13 @@ constexpr Shape adv_shape(int P, bool fp32) {
     if (P <= 48) {
         s.T = 64;
         s.MINB = fp32 ? 8 : 6;
+    } else if (fp32 && P <= 216) {
+        s.NR = 4;
+        s.T = P <= 108 ? 96 : (P <= 162 ? 128 : 192);
+        s.MINB = s.T == 96 ? 7 : (s.T == 128 ? 5 : 4);
     } else if (fp32) {
         s.T = larger > 24 ? 192 : 96;
-        s.MINB = larger > 24 ? 2 : (larger >= 18 ? 5 : (P == 192 ? 8 : 6));
+        s.MINB = larger > 24 ? 2 : (larger >= 18 ? 5 : 6);
     } else {
         s.T = P > 216 && P < 384 ? 128 : 96;
         s.MINB = s.T == 128 || P >= 384 ? 3 : (larger <= 9 || P <= 144 ? 5 : 4);
@@ -66,25 +72,27 @@ constexpr Shape adv_shape(int P, bool fp32) {
     return s;
 }
 
-// Smagorinsky (P1 = 2 k1max + 2).  One row per block above 128 points (double: 144):
-// the carried values of a point take 13 registers (26), so small blocks are what keeps
-// several of them on an SM (256 points, single: one row and 64 threads 0.153 ms, two
-// rows and 128 threads 0.171 ms; 256^2 x 64).  Single-precision rows of an odd number
-// of modes go in pairs, which fill the 16-byte units of the bulk copies.
+// Smagorinsky (P1 = 2 k1max + 2).  Single precision: two rows per block, one above 288
+// points, and one thread per task of the last forward pass (four lines a row of B tasks:
+// 64 points 64 / 96 / 128 threads 111 / 138 / 130 us at 64^2 x 768; 256 points, one row and
+// 64 threads 280, two rows and 128 threads 240 us at 256^2 x 128).  Double precision, whose
+// carried values take 26 registers a point: one row above 144 points.
 constexpr Shape sgs_shape(int P, bool fp32) {
     Shape s;
     if (P < 12 || P > (fp32 ? 512 : 324)) return s;
     factor(s, P, fp32, 2);
     if (P == 96 && fp32) s.A = 6, s.B = 16;
     if (!s.A) return s;
+    const int larger = s.A > s.B ? s.A : s.B;
     if (fp32) {
-        s.NR = P <= 128 || P % 4 ? 2 : 1;
-        s.T = P <= 32 ? 64 : (s.NR == 1 && P <= 288 ? 64 : (P < 90 ? 96 : 128));
-        s.MINB = s.NR == 1 ? (s.T == 64 ? 7 : 3) : (P > 128 ? 3 : (s.T == 128 ? 4 : (s.T == 96 ? 5 : 8)));
+        s.NR = P <= 288 || P % 4 ? 2 : 1;
+        s.T = (4 * s.NR * s.B + 31) / 32 * 32;
+        if (s.T > 160) s.T = 160;
+        s.MINB = s.T == 32 ? 16 : (s.T == 64 ? 8 : (s.T == 96 ? 5 : (s.T == 160 || s.NR == 1 ? 3 : (P == 128 ? 5 : 4))));
     } else {
         s.NR = P <= 144 ? 2 : 1;
-        s.T = P <= 48 ? 64 : 96;
-        s.MINB = s.T == 64 ? 6 : 4;
+        s.T = P <= 72 ? 64 : 96;
+        s.MINB = s.T == 96 ? 4 : (larger <= 8 ? 8 : 6);
     }
     return s;
 }

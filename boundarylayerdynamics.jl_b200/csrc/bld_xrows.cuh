@@ -90,7 +90,7 @@ struct AdvCarry {
     R w, o1, o2, c;   // w, vort1, vort2 on the I layer below and vort2 u - vort1 v there
 };
 
-// grid (P2 / NR, nchunks, members), block T threads.  SEPF: the forward lines have
+// grid (ceil(P2 / NR), nchunks, members), block T threads.  SEPF: the forward lines have
 // their own buffer, so the stores of layer j share a barrier interval with inverse
 // pass 1 of layer j + 1.  Needs 3 k1max < P (middle third of the spectrum empty)
 // where A is a multiple of 3.
@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(T, MINB) k_adv_row(XArgs a) {
     C* Fw = SEPF ? reinterpret_cast<C*>(p) : Ln;
     const C* Min = reinterpret_cast<const C*>(a.min) + (long long)m * a.min_mstride;
     C* Mout = reinterpret_cast<C*>(a.mout) + (long long)m * a.mout_mstride;
-    const unsigned row_bytes = (unsigned)(NR * K1 * csz);
+    const int nr = min(NR, a.P2 - y0);   // rows of this block (even); the others are not stored
+    const unsigned row_bytes = (unsigned)(nr * K1 * csz);
     // staged slots: u, v, vort3 (C); w, vort1, vort2 (I) = mixed terms 0, 1, 5, 2, 3, 4
     auto issue = [&](int j) {
         const int nslots = (j < n3 - 1) ? 6 : 3;
@@ -258,14 +259,14 @@ __global__ void __launch_bounds__(T, MINB) k_adv_row(XArgs a) {
         // ---- forward pass 2, unpacking and the store of the modes
         for (int l0 = lf0 + (threadIdx.x >> 5) * LW; l0 < lf1; l0 += (T / 32) * LW) {
             const int lane = threadIdx.x & 31, g = lane / B, kp = lane % B;
-            const bool ok = g < LW && l0 + g < lf1;
-            const int L = ok ? l0 + g : l0;
+            const int L = g < LW && l0 + g < lf1 ? l0 + g : l0;
+            const bool ok = L == l0 + g && (L < NR ? L : 2 * (L - NR)) < nr;
             const C* src = Fw + (SEPF ? L : (L < NR ? 3 * L : 6 * (L - NR) + 1)) * LS + kp;
             C x[A];
 #pragma unroll
             for (int t = 0; t < A; ++t) x[t] = src[t * BS];
             dft<R, A, -1>(x);
-            const int partner = ok && kp ? lane + B - 2 * kp : lane;
+            const int partner = g < LW && kp ? lane + B - 2 * kp : lane;
             C *oa, *ob;
             if (L < NR) {
                 oa = mrow_w(Mout, a, 0, j, y0 + L) + kp;

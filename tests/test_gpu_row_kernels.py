@@ -47,7 +47,7 @@ def _state(om, seed):
 
 @pytest.mark.parametrize("res", [(12, 12, 3), (18, 16, 5), (23, 30, 4), (50, 42, 7), (70, 54, 6), (98, 16, 9),
                                  (100, 84, 17), (108, 10, 4), (150, 14, 5), (192, 12, 6), (252, 16, 4),
-                                 (256, 18, 5), (320, 12, 4)])
+                                 (256, 18, 5), (320, 12, 4), (64, 35, 5)])
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-5)])
 def test_les_rates(oracle, BLD, res, precision, tol):
     om, gm = _les(oracle, res), _les(BLD, res, precision=precision)
