@@ -173,12 +173,16 @@ int set_smem_limits() {
     CUDA_TRY(cudaFuncSetAttribute(k_x_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(k_project_seg<8, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     // dynamic shared memory of k_project_tile: at most 200 KB (project_tile_ok)
-    CUDA_TRY(cudaFuncSetAttribute(k_project_tile<8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(k_project_tile<8, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(k_project_tile<16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(k_project_tile<16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(k_project_tile<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(k_project_tile<16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+#define BLD_SET_TILE(L, N)                                                                                           \
+    CUDA_TRY(cudaFuncSetAttribute(k_project_tile<L, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));   \
+    CUDA_TRY(cudaFuncSetAttribute(k_project_tile<L, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    BLD_SET_TILE(8, 4)
+    BLD_SET_TILE(8, 8)
+    BLD_SET_TILE(8, 16)
+    BLD_SET_TILE(16, 4)
+    BLD_SET_TILE(16, 8)
+    BLD_SET_TILE(16, 16)
+#undef BLD_SET_TILE
     // k_project_pipe: at most 200 KB as well (project_pipe_ok)
     CUDA_TRY(cudaFuncSetAttribute(k_project_pipe<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(k_project_pipe<8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -548,7 +552,7 @@ struct TuneKey {
 };
 struct TuneVal {
     Space adv, sgs;
-    int proj_variant, proj_tile, proj_pipe;
+    int proj_variant, proj_tile, proj_pipe, proj_euler;
 };
 std::mutex g_tune_mutex;
 std::map<TuneKey, TuneVal> g_tune_cache;
@@ -557,7 +561,8 @@ TuneKey tune_key(const bld_handle* h) {
     // any kernel-family switch in the environment makes its own entry
     int env = 0;
     for (const char* v : {"BLD_X_KERNEL", "BLD_Y_KERNEL", "BLD_XW_MINB", "BLD_PROJ_VARIANT", "BLD_X_LINES",
-                          "BLD_SGS_X_KERNEL", "BLD_X2_VARIANT", "BLD_PROJ_TILE", "BLD_PROJ_PIPE", "BLD_SGS_X2_VARIANT"}) {
+                          "BLD_SGS_X_KERNEL", "BLD_X2_VARIANT", "BLD_PROJ_TILE", "BLD_PROJ_PIPE", "BLD_SGS_X2_VARIANT",
+                          "BLD_PROJ_EULER"}) {
         const char* e = getenv(v);
         env = env * 31 + (e ? (int)(std::hash<std::string>{}(e) % 1000003) + 1 : 0);
     }
@@ -600,6 +605,7 @@ int autotune(bld_handle* h) {
             h->proj_variant = it->second.proj_variant;
             h->proj_tile = it->second.proj_tile;
             h->proj_pipe = it->second.proj_pipe;
+            h->proj_euler = it->second.proj_euler;
             return BLD_OK;
         }
     }
@@ -612,6 +618,7 @@ int autotune(bld_handle* h) {
         v.proj_variant = h->proj_variant;
         v.proj_tile = h->proj_tile;
         v.proj_pipe = h->proj_pipe;
+        v.proj_euler = h->proj_euler;
         g_tune_cache[key] = v;
     }
     return BLD_OK;
@@ -899,6 +906,21 @@ int autotune_impl(bld_handle* h) {
             }
         h->proj_tile = btile;
         h->proj_pipe = bpipe;
+        // the Euler stage that starts a step: the chosen variant against the tile kernel
+        // (a forced variant keeps its own; BLD_PROJ_EULER = 0 or 1 keeps one)
+        const char* pe = getenv("BLD_PROJ_EULER");
+        const int only_e = (pe && pe[0]) ? atoi(pe) : -1;
+        h->proj_euler = btile && only_e == 1;
+        if (btile && only_v < 0 && only_e < 0) {
+            float te[2] = {0, 0};
+            for (int e = 0; e < 2; ++e) {
+                h->proj_euler = e;
+                BLD_TRY(time_launches(h, [&] {
+                    return enqueue_project(h, S_EULER, 1e-4, h->u, nullptr, h->du, nullptr, h->io, 0, B);
+                }, 3, &te[e]));
+            }
+            h->proj_euler = te[1] < te[0];
+        }
         const char* v = getenv("BLD_VERBOSE");
         if (v && v[0] && v[0] != '0') fprintf(stderr, "bld autotune projection: variant %d, tile %d, persistent %d\n", bv, btile, bpipe);
     }
@@ -1009,13 +1031,13 @@ int enqueue_project(bld_handle* h, int kind, double dt, const double2* u, const 
     const bool any_mean = h->cfg.mean[0] || h->cfg.mean[1];
     if (!a.pressure && !any_mean && kind == S_NONE && out == u) return BLD_OK;
     const int n3 = h->g.n3;
-    if (kind == S_NONE && h->proj_tile && project_tile_ok(h, h->proj_tile)) {
+    if ((kind == S_NONE || (kind == S_EULER && h->proj_euler)) && h->proj_tile && project_tile_ok(h, h->proj_tile)) {
         const int ln = h->proj_tile, lmax = n3 <= 128 ? 8 : 16;
         CUtensorMap umap, gmap;
         BLD_TRY(project_tmaps(h, u, ln, &umap, &gmap));
         dim3 grid((unsigned)((h->g.F + ln - 1) / ln), nm);
         dim3 block(ln, std::max(1, std::min(16, (n3 + lmax - 1) / lmax)));
-        if (h->proj_pipe && project_pipe_ok(h, ln)) {
+        if (kind == S_NONE && h->proj_pipe && project_pipe_ok(h, ln)) {
             if (lmax == 8 && ln == 4) return launch_project_pipe<8, 4>(h, a, nm, umap, gmap);
             if (lmax == 8 && ln == 8) return launch_project_pipe<8, 8>(h, a, nm, umap, gmap);
             if (lmax == 8) return launch_project_pipe<8, 16>(h, a, nm, umap, gmap);
@@ -1024,12 +1046,18 @@ int enqueue_project(bld_handle* h, int kind, double dt, const double2* u, const 
             return launch_project_pipe<16, 16>(h, a, nm, umap, gmap);
         }
         const size_t sm = project_tile_smem(n3, ln);
-        if (lmax == 8 && ln == 4) k_project_tile<8, 4><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag);
-        else if (lmax == 8 && ln == 8) k_project_tile<8, 8><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag);
-        else if (lmax == 8) k_project_tile<8, 16><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag);
-        else if (ln == 4) k_project_tile<16, 4><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag);
-        else if (ln == 8) k_project_tile<16, 8><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag);
-        else k_project_tile<16, 16><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag);
+#define BLD_TILE(L, N)                                                                                          \
+    if (lmax == L && ln == N) {                                                                                \
+        if (kind == S_EULER) k_project_tile<L, N, true><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag); \
+        else k_project_tile<L, N><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag);                      \
+    }
+        BLD_TILE(8, 4)
+        BLD_TILE(8, 8)
+        BLD_TILE(8, 16)
+        BLD_TILE(16, 4)
+        BLD_TILE(16, 8)
+        BLD_TILE(16, 16)
+#undef BLD_TILE
         CUDA_TRY(cudaGetLastError());
         return BLD_OK;
     }

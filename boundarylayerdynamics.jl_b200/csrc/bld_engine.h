@@ -213,6 +213,7 @@ struct bld_handle {
     std::map<std::pair<int, double>, cudaGraph_t> graph_src;   // kept for ensemble parent graphs
     std::map<std::vector<const void*>, cudaGraphExec_t> ens_graphs;  // parent graphs led by this handle
     size_t bytes = 0;
+    int proj_euler = 0;          // 1: the Euler stage of a step by k_project_tile too (autotuned)
     cudaStream_t side = nullptr;   // second branch of the right-hand side (with both physical spaces)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 };

@@ -1,4 +1,5 @@
-// Pressure projection of a stage value that is already stored (k_project_tile).
+// Pressure projection of a stage value that is already stored (k_project_tile), and
+// of the Euler stage u^n + dt du that starts a step (EULER).
 //
 // Same arithmetic as k_project_seg for the stage kind S_NONE (div!,
 // src/processes/pressure.jl:368-378; the LDL^T sweeps of ldiv!, :106-165;
@@ -26,19 +27,19 @@
 // values per component tile: n3 LN rounded up to 8 (128 bytes), so that every
 // TMA destination starts on a 128-byte boundary whatever n3 and LN are
 __host__ __device__ constexpr int project_tile_stride(int n3, int LN) { return (n3 * LN + 7) / 8 * 8; }
-// bytes: alignment slack, the barrier, the three components, gamma
+// bytes: alignment slack, the barrier, the three components, gamma, the two tables
 __host__ __device__ constexpr int project_tile_smem(int n3, int LN) {
-    return 128 + 128 + 3 * project_tile_stride(n3, LN) * 16 + n3 * LN * 8;
+    return 128 + 128 + 3 * project_tile_stride(n3, LN) * 16 + n3 * LN * 8 + 2 * n3 * 8;
 }
 
 // bytes of one stage of k_project_pipe (the three component tiles and gamma),
 // rounded to 128; dynamic shared memory of k_project_pipe: slack, the two
-// barriers, two stages
+// barriers, two stages, the tables
 __host__ __device__ constexpr int project_stage_bytes(int n3, int LN) {
     return (3 * project_tile_stride(n3, LN) * 16 + n3 * LN * 8 + 127) / 128 * 128;
 }
 __host__ __device__ constexpr int project_pipe_smem(int n3, int LN) {
-    return 128 + 128 + 2 * project_stage_bytes(n3, LN);
+    return 128 + 128 + 2 * project_stage_bytes(n3, LN) + 2 * n3 * 8;
 }
 
 // Issues the TMA copies of the LN columns from c0 of member m into one stage
@@ -54,12 +55,26 @@ __device__ __forceinline__ void project_tile_issue(const CUtensorMap* umap, cons
     tma_load_2d(reinterpret_cast<double*>(tile + 3 * FS), gmap, c0, 0, bar);
 }
 
+// The layer tables of the solve in shared memory: alpha_i[n3 - 1] (and a zero), then
+// 1 / alpha_c[n3].  Read from global memory, they were a chain of cache latencies in
+// every sweep (192^2 x 96 49 -> 41 us with them here and the segments of full length
+// unrolled; 256^2 x 256 271 -> 209 us; 24 x 64^2 x 32 41 -> 30 us).
+__device__ __forceinline__ void project_tables(double* tab, const ProjArgs& a, int tid, int nthreads) {
+    const int n = a.g.n3;
+    for (int i = tid; i < n; i += nthreads) {
+        tab[i] = i < n - 1 ? __ldg(a.alpha_i + i) : 0.0;
+        tab[n + i] = __ldg(a.inv_alpha_c + i);
+    }
+}
+
 // The solve of one staged tile (columns c0 .. c0 + LN - 1 of member m), writing
 // u + grad p to a.out; every thread of the block calls it, and it ends after a
-// barrier that follows the block's last read of the tile.
-template <int LMAX, int LN>
-__device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const double2* tile, int FS, int c0, int m,
-                                                   double2 (*sP)[LN], double (*sQ)[LN]) {
+// barrier that follows the block's last read of the tile.  FULL: every segment has
+// LMAX layers.  EULER: the tile holds u^n, and the stage value u^n + dt du
+// (src/ODEMethods.jl:101,143,157) is formed in it first.
+template <int LMAX, int LN, bool FULL, bool EULER>
+__device__ __forceinline__ void project_tile_body(const ProjArgs& a, double2* tile, const double* tab, int FS, int c0,
+                                                  int m, double2 (*sP)[LN], double (*sQ)[LN]) {
     const Geo& g = a.g;
     const int n = g.n3;
     const long long F = g.F;
@@ -67,9 +82,11 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     const int NS = blockDim.y, s = threadIdx.y, lane = threadIdx.x;
     const int c = c0 + lane;
     const bool valid = c < F;
-    const int L = (n + NS - 1) / NS;
+    const int L = FULL ? LMAX : (n + NS - 1) / NS;
     const int z0 = min(n, s * L), z1 = min(n, z0 + L);
-    const int len = z1 - z0;
+    const int len = FULL ? LMAX : z1 - z0;
+    const double* sai = tab;
+    const double* sic = tab + n;
     const long long mb = (long long)m * g.mstride;
     const long long o1 = mb, o2 = mb + (long long)n * F, o3 = mb + 2LL * n * F;
     const int cc = valid ? c : 0;
@@ -77,6 +94,24 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     const bool mean_mode = (c == 0);
     const double e1 = a.d1[k1], e2 = a.d2[j];
     auto U = [&](int f, int z) -> double2 { return tile[f * FS + z * LN + lane]; };
+    if constexpr (EULER) {
+        const double2* du = a.du + mb + cc;
+#pragma unroll 1
+        for (int f = 0; f < 3; ++f) {
+            double2 D[LMAX];
+#pragma unroll
+            for (int q = 0; q < LMAX; ++q)
+                if ((FULL || q < len) && (f < 2 || z0 + q < n - 1))
+                    D[q] = __ldg(du + (long long)(f * n + z0 + q) * F);
+#pragma unroll
+            for (int q = 0; q < LMAX; ++q)
+                if ((FULL || q < len) && (f < 2 || z0 + q < n - 1)) {
+                    double2& t = tile[f * FS + (z0 + q) * LN + lane];
+                    t = make_double2(t.x + a.dt * D[q].x, t.y + a.dt * D[q].y);
+                }
+        }
+        __syncthreads();   // the segment above reads this one's last w
+    }
     double2 wprev = make_double2(0.0, 0.0);
     if (z0 > 0 && len > 0) wprev = U(2, z0 - 1);
     double2 X[LMAX];
@@ -85,10 +120,10 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
 #pragma unroll
     for (int q = 0; q < LMAX; ++q) {
         const int z = z0 + q;
-        if (q < len) {
+        if (FULL || q < len) {
             const double2 uz = U(0, z), vz = U(1, z);
-            const double2 wz = (z < n - 1) ? U(2, z) : make_double2(0.0, 0.0);
-            const double h = a.inv_alpha_c[z];
+            const double2 wz = U(2, z);   // zero in the last layer (the copy's fill past the state)
+            const double h = sic[z];
             double2 val;
             val.x = (-e1 * uz.y) * h + (-e2 * vz.y) * h;
             val.y = (e1 * uz.x) * h + (e2 * vz.x) * h;
@@ -111,9 +146,9 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
                 Y[q] = 0.0;
             } else if (q == 0) {
                 X[q] = make_double2(gm * val.x, gm * val.y);
-                Y[q] = -gm * a.alpha_i[z - 1];
+                Y[q] = -gm * sai[z - 1];
             } else {
-                const double be = a.alpha_i[z - 1];
+                const double be = sai[z - 1];
                 X[q] = make_double2(gm * (val.x - be * X[q - 1].x), gm * (val.y - be * X[q - 1].y));
                 Y[q] = -gm * be * Y[q - 1];
             }
@@ -124,7 +159,10 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     {
         double2 pe = make_double2(0.0, 0.0);
         double qe = 1.0;
-        if (len > 0) {
+        if (FULL) {
+            pe = X[LMAX - 1];
+            qe = Y[LMAX - 1];
+        } else if (len > 0) {
 #pragma unroll
             for (int q = 0; q < LMAX; ++q)
                 if (q < len) {
@@ -137,6 +175,7 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     }
     __syncthreads();
     double2 bin = make_double2(0.0, 0.0);
+#pragma unroll 4
     for (int t = 0; t < s; ++t) {
         const double2 pe = sP[t][lane];
         const double qe = sQ[t][lane];
@@ -146,17 +185,17 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     // ---- b_z, then the segment-local backward sweep
 #pragma unroll
     for (int q = 0; q < LMAX; ++q)
-        if (q < len) X[q] = make_double2(X[q].x + Y[q] * bin.x, X[q].y + Y[q] * bin.y);
+        if (FULL || q < len) X[q] = make_double2(X[q].x + Y[q] * bin.x, X[q].y + Y[q] * bin.y);
 #pragma unroll
     for (int qq = 0; qq < LMAX; ++qq) {
         const int q = LMAX - 1 - qq;
-        if (q >= len) continue;
+        if (!FULL && q >= len) continue;
         const int z = z0 + q;
         if (z == n - 1) {
             Y[q] = 0.0;   // p_{n-1} = b_{n-1}
         } else {
-            const double cz = gt[z * LN + lane] * a.alpha_i[z];
-            if (q == len - 1 || q == LMAX - 1) {
+            const double cz = gt[z * LN + lane] * sai[z];
+            if (q == LMAX - 1 || (!FULL && q == len - 1)) {
                 Y[q] = -cz;
             } else {
                 X[q] = make_double2(X[q].x - cz * X[q + 1].x, X[q].y - cz * X[q + 1].y);
@@ -167,7 +206,7 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     {
         double2 ps = make_double2(0.0, 0.0);
         double hs = 1.0;
-        if (len > 0) {
+        if (FULL || len > 0) {
             ps = X[0];
             hs = Y[0];
         }
@@ -176,6 +215,7 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     }
     __syncthreads();
     double2 pout = make_double2(0.0, 0.0);
+#pragma unroll 4
     for (int t = NS - 1; t > s; --t) {
         const double2 ps = sP[t][lane];
         const double hs = sQ[t][lane];
@@ -184,16 +224,16 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     // ---- pressure and gradient
 #pragma unroll
     for (int q = 0; q < LMAX; ++q)
-        if (q < len) X[q] = make_double2(X[q].x + Y[q] * pout.x, X[q].y + Y[q] * pout.y);
+        if (FULL || q < len) X[q] = make_double2(X[q].x + Y[q] * pout.x, X[q].y + Y[q] * pout.y);
 #pragma unroll
     for (int q = 0; q < LMAX; ++q) {
         const int z = z0 + q;
-        if (q < len && valid) {
+        if ((FULL || q < len) && valid) {
             const double2 pz = X[q];
             double2 pn = pout;
 #pragma unroll
             for (int rr = 0; rr < LMAX; ++rr)
-                if (rr == q + 1 && rr < len) pn = X[rr];
+                if (rr == q + 1 && (FULL || rr < len)) pn = X[rr];
             double2 u = U(0, z), v = U(1, z);
             u.x += e1 * pz.y;
             u.y += -e1 * pz.x;
@@ -203,7 +243,7 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
             a.out[o2 + z * F + c] = v;
             if (z < n - 1) {
                 double2 w = U(2, z);
-                const double ai = a.alpha_i[z];
+                const double ai = sai[z];
                 w.x += -1.0 * (-ai * pz.x + ai * pn.x);
                 w.y += -1.0 * (-ai * pz.y + ai * pn.y);
                 a.out[o3 + z * F + c] = w;
@@ -224,7 +264,16 @@ __device__ __forceinline__ void project_tile_solve(const ProjArgs& a, const doub
     }
 }
 
-template <int LMAX, int LN>
+template <int LMAX, int LN, bool EULER>
+__device__ __forceinline__ void project_tile_solve(const ProjArgs& a, double2* tile, const double* tab, int FS, int c0,
+                                                   int m, double2 (*sP)[LN], double (*sQ)[LN]) {
+    if (a.g.n3 == LMAX * (int)blockDim.y)
+        project_tile_body<LMAX, LN, true, EULER>(a, tile, tab, FS, c0, m, sP, sQ);
+    else
+        project_tile_body<LMAX, LN, false, EULER>(a, tile, tab, FS, c0, m, sP, sQ);
+}
+
+template <int LMAX, int LN, bool EULER = false>
 __global__ void __launch_bounds__(LN * 32) k_project_tile(ProjArgs a, const __grid_constant__ CUtensorMap umap,
                                                         const __grid_constant__ CUtensorMap gmap, int* flag) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -235,7 +284,8 @@ __global__ void __launch_bounds__(LN * 32) k_project_tile(ProjArgs a, const __gr
     uint64_t* bar = reinterpret_cast<uint64_t*>(base);
     const int n = a.g.n3;
     const int FS = project_tile_stride(n, LN);
-    double2* tile = reinterpret_cast<double2*>(base + 128);   // [3][FS >= n LN], then gamma
+    double2* tile = reinterpret_cast<double2*>(base + 128);   // [3][FS >= n LN], then gamma, the tables
+    double* tab = reinterpret_cast<double*>(tile + 3 * FS) + n * LN;
     const int tid = threadIdx.y * LN + threadIdx.x;
     const int c0 = blockIdx.x * LN;
     const int m = a.m0 + blockIdx.y;
@@ -250,6 +300,7 @@ __global__ void __launch_bounds__(LN * 32) k_project_tile(ProjArgs a, const __gr
         prefetch_tmap(&gmap);
         project_tile_issue<LN>(&umap, &gmap, tile, FS, n, c0, m, bar);
     }
+    project_tables(tab, a, tid, blockDim.x * blockDim.y);   // published by the barrier below
     const long long wait_limit = g_bld_wait_limit;
     const bool arrived = mbar_wait_bounded(bar, 0, wait_limit);
     if (__syncthreads_or(!arrived)) {
@@ -259,7 +310,7 @@ __global__ void __launch_bounds__(LN * 32) k_project_tile(ProjArgs a, const __gr
         }
         return;
     }
-    project_tile_solve<LMAX, LN>(a, tile, FS, c0, m, sP, sQ);
+    project_tile_solve<LMAX, LN, EULER>(a, tile, tab, FS, c0, m, sP, sQ);
 }
 
 // persistent form: grid (blocks, 1), block (LN, NS), dynamic shared memory
@@ -279,11 +330,13 @@ __global__ void __launch_bounds__(LN * 32) k_project_pipe(ProjArgs a, int nm, co
     const int tid = threadIdx.y * LN + threadIdx.x;
     const int ntiles = (int)((a.g.F + LN - 1) / LN);
     const int total = ntiles * nm;
+    double* tab = reinterpret_cast<double*>(base + 128 + 2 * SB);
     const int step = (int)gridDim.x;
     // this block's first active item
     int it = blockIdx.x;
     while (it < total && a.active && !a.active[a.m0 + it / ntiles]) it += step;
     if (it >= total) return;
+    project_tables(tab, a, tid, blockDim.x * blockDim.y);
     if (tid == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -319,7 +372,7 @@ __global__ void __launch_bounds__(LN * 32) k_project_pipe(ProjArgs a, int nm, co
             }
             return;
         }
-        project_tile_solve<LMAX, LN>(a, reinterpret_cast<const double2*>(base + 128 + s * SB), FS, c0, m, sP, sQ);
+        project_tile_solve<LMAX, LN, false>(a, reinterpret_cast<double2*>(base + 128 + s * SB), tab, FS, c0, m, sP, sQ);
         it = nx;
     }
 }
