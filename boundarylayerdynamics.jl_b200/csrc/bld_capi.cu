@@ -9,6 +9,7 @@
 #include <tuple>
 
 #include "bld_engine.h"
+#include "bld_hostcopy.h"
 #include "bld_project_tile.cuh"
 #include "bld_yline.h"
 
@@ -1388,6 +1389,7 @@ void free_handle(bld_handle* h) {
     if (h->ev_join) cudaEventDestroy(h->ev_join);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
+    HostCopy::get().drop_user();
     delete h;
 }
 
@@ -1429,6 +1431,7 @@ int32_t bld_create(const bld_config* cfg, bld_handle** out) {
     CUDA_TRY(cudaSetDevice(cfg->device));
     BLD_TRY(set_smem_limits());
     bld_handle* h = new bld_handle();
+    HostCopy::get().add_user();   // dropped by free_handle
     h->cfg = *cfg;
     h->cfg.dx3_c = h->cfg.dx3_i = h->cfg.x3_c = h->cfg.x3_i = nullptr;  // caller memory: copied below
     h->cfg.member_cs = h->cfg.member_z0_lower = h->cfg.member_source1 = nullptr;
@@ -1445,7 +1448,7 @@ int32_t bld_create(const bld_config* cfg, bld_handle** out) {
     g.mstride = (long long)(3 * g.n3 - 1) * g.F;
     const int n3 = g.n3, K1 = g.K1, K2 = g.K2, B = h->B;
     if (cudaGetSymbolAddress((void**)&h->wait_limit, g_bld_wait_limit) != cudaSuccess) {
-        delete h;
+        free_handle(h);
         return fail(BLD_ERR_CUDA, "cudaGetSymbolAddress failed");
     }
     auto bail = [&](int code) {
@@ -1654,9 +1657,9 @@ static int copy_fields_h2d(bld_handle* h, double2* base, int m, const double* v1
     const Geo& g = h->g;
     double2* dst = base + (size_t)m * g.mstride;
     const size_t nc = (size_t)g.n3 * g.F, ni = (size_t)(g.n3 - 1) * g.F;
-    CUDA_TRY(cudaMemcpyAsync(dst, v1, nc * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(cudaMemcpyAsync(dst + nc, v2, nc * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(cudaMemcpyAsync(dst + 2 * nc, v3, ni * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(HostCopy::get().copy(dst, v1, nc * sizeof(double2), true, h->stream, h->device));
+    CUDA_TRY(HostCopy::get().copy(dst + nc, v2, nc * sizeof(double2), true, h->stream, h->device));
+    CUDA_TRY(HostCopy::get().copy(dst + 2 * nc, v3, ni * sizeof(double2), true, h->stream, h->device));
     return BLD_OK;
 }
 
@@ -1664,9 +1667,9 @@ static int copy_fields_d2h(bld_handle* h, const double2* base, int m, double* v1
     const Geo& g = h->g;
     const double2* src = base + (size_t)m * g.mstride;
     const size_t nc = (size_t)g.n3 * g.F, ni = (size_t)(g.n3 - 1) * g.F;
-    CUDA_TRY(cudaMemcpyAsync(v1, src, nc * sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(cudaMemcpyAsync(v2, src + nc, nc * sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(cudaMemcpyAsync(v3, src + 2 * nc, ni * sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(HostCopy::get().copy(v1, src, nc * sizeof(double2), false, h->stream, h->device));
+    CUDA_TRY(HostCopy::get().copy(v2, src + nc, nc * sizeof(double2), false, h->stream, h->device));
+    CUDA_TRY(HostCopy::get().copy(v3, src + 2 * nc, ni * sizeof(double2), false, h->stream, h->device));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return BLD_OK;
 }
@@ -2203,8 +2206,8 @@ int32_t bld_set_field_physical(bld_handle* h, int32_t m, int32_t field, const do
     if (!h->pd_buf) return fail(BLD_ERR_INVALID_CONFIG, "default physical size is not an even 2^a*3^b");
     CUDA_TRY(cudaSetDevice(h->device));
     const int nz = field == 2 ? h->g.n3 - 1 : h->g.n3;
-    CUDA_TRY(cudaMemcpyAsync(h->pd_buf, values, (size_t)nz * h->Pd2 * h->Pd1 * sizeof(double), cudaMemcpyHostToDevice,
-                             h->stream));
+    CUDA_TRY(HostCopy::get().copy(h->pd_buf, values, (size_t)nz * h->Pd2 * h->Pd1 * sizeof(double), true, h->stream,
+                                  h->device));
     BLD_TRY(set_field_from_pd(h, m, field));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return BLD_OK;
@@ -2285,7 +2288,7 @@ int32_t bld_get_field_physical(bld_handle* h, int32_t m, int32_t field, double* 
     const int nz = field == 2 ? h->g.n3 - 1 : h->g.n3;
     const int P1 = h->Pd1, P2 = h->Pd2;
     BLD_TRY(physical_field_dev(h, m, field, P1, P2, (double2*)h->pd_mixed, (double*)h->pd_buf));
-    CUDA_TRY(cudaMemcpyAsync(values, h->pd_buf, (size_t)nz * P2 * P1 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(HostCopy::get().copy(values, h->pd_buf, (size_t)nz * P2 * P1 * sizeof(double), false, h->stream, h->device));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return BLD_OK;
 }
