@@ -10,6 +10,7 @@
 
 #include "bld_engine.h"
 #include "bld_hostcopy.h"
+#include "bld_launch_util.cuh"
 #include "bld_project_tile.cuh"
 #include "bld_yline.h"
 
@@ -31,6 +32,12 @@ int bld::fail(int code, const char* fmt, ...) {
 }
 
 namespace {
+
+// BLD_NO_OVERLAP=1 launches every kernel after the one before it has ended
+bool overlap_on() {
+    const char* e = getenv("BLD_NO_OVERLAP");
+    return !(e && e[0] && e[0] != '0');
+}
 
 // k_project_tile applies: the pressure solve with <= 256 layers, an even number
 // of modes per layer (gamma rows are 16-byte multiples for the TMA map) and
@@ -72,8 +79,8 @@ int launch_project_pipe(bld_handle* h, const ProjArgs& a, int nm, const CUtensor
     }
     const long long items = (h->g.F + LN - 1) / LN * (long long)nm;
     const int blocks = (int)std::min<long long>(items, (long long)std::max(1, per_sm) * nsm);
-    k_project_pipe<LMAX, LN><<<blocks, block, sm, h->stream>>>(a, nm, umap, gmap, h->flag);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(bld_util::launch(k_project_pipe<LMAX, LN>, dim3(blocks), block, sm, h->stream,
+                              h->overlap && overlap_on(), a, nm, umap, gmap, h->flag));
     return BLD_OK;
 }
 
@@ -213,6 +220,7 @@ int enqueue_inv_y_R(bld_handle* h, int sp, const double2* state, int m0, int nm)
     ia.active = h->mask_on ? h->active : nullptr;
     ia.plan = s.plan2;
     ia.tw = twp(h, s.P2, sizeof(R) == 4);
+    ia.overlap = h->overlap && overlap_on();
     if (sp == 0) {  // u, v, w, vort1, vort2, vort3 (src/processes/momentum_advection.jl:40-41)
         const int op[6] = {T_DIRECT, T_DIRECT, T_DIRECT, T_VORT1, T_VORT2, T_VORT3};
         const int fl[6] = {0, 1, 2, 0, 0, 0};
@@ -282,6 +290,7 @@ int enqueue_x_R(bld_handle* h, int sp, int m0, int nm) {
     xa.active = h->mask_on ? h->active : nullptr;
     xa.d1 = h->d1;
     xa.wait_limit = h->wait_limit;
+    xa.overlap = h->overlap && overlap_on();
     if (s.xrow) return launch_row(h, s, xa, nm);
     if (sp == 0) {
         return launch_adv_family<R>(h, s, xa, nm);
@@ -348,6 +357,7 @@ int enqueue_fwd_y_R(bld_handle* h, int sp, bool first, bool last, const double2*
     fa.active = h->mask_on ? h->active : nullptr;
     fa.plan = s.plan2;
     fa.tw = twp(h, s.P2, sizeof(R) == 4);
+    fa.overlap = h->overlap && overlap_on();
     if (sf) {
         if (s.fwd.all && !s.yl) return fail(BLD_ERR_INVALID_CONFIG, "stage fusion needs the per-term forward y kernel");
         fa.fuse = 1;
@@ -515,22 +525,28 @@ std::vector<YCfg> y_candidates(const bld_handle* h, const Space& s, int lines_pe
     return out;
 }
 
-// average device time of `iters` launches of fn after one warm-up launch
+// average device time of `fn` after one warm-up launch, over `iters` launches or, for
+// short kernels, as many (up to 40) as take 0.2 ms: the events tick in steps of about 2 us
 template <typename F>
 int time_launches(bld_handle* h, F&& fn, int iters, float* ms) {
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
     int st = fn();
-    if (st == BLD_OK && cudaEventRecord(e0, h->stream) != cudaSuccess) st = BLD_ERR_CUDA;
-    for (int i = 0; i < iters && st == BLD_OK; ++i) st = fn();
-    if (st == BLD_OK && cudaEventRecord(e1, h->stream) != cudaSuccess) st = BLD_ERR_CUDA;
-    if (st == BLD_OK && cudaEventSynchronize(e1) != cudaSuccess) st = BLD_ERR_CUDA;
     float t = 0;
-    if (st == BLD_OK) cudaEventElapsedTime(&t, e0, e1);
+    for (int round = 0; round < 2 && st == BLD_OK; ++round) {
+        if (st == BLD_OK && cudaEventRecord(e0, h->stream) != cudaSuccess) st = BLD_ERR_CUDA;
+        for (int i = 0; i < iters && st == BLD_OK; ++i) st = fn();
+        if (st == BLD_OK && cudaEventRecord(e1, h->stream) != cudaSuccess) st = BLD_ERR_CUDA;
+        if (st == BLD_OK && cudaEventSynchronize(e1) != cudaSuccess) st = BLD_ERR_CUDA;
+        if (st == BLD_OK) cudaEventElapsedTime(&t, e0, e1);
+        t /= iters;
+        if (t * iters >= 0.1f) break;
+        iters = std::max(iters, std::min(40, (int)(0.2f / std::max(t, 0.002f))));
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    *ms = t / iters;
+    *ms = t;
     return st == BLD_ERR_CUDA ? fail(BLD_ERR_CUDA, "autotune timing failed") : st;
 }
 
@@ -930,10 +946,28 @@ int autotune_impl(bld_handle* h) {
     return BLD_OK;
 }
 
+// Whether the advection's inverse y pass has clearly more blocks than the device holds at
+// once.  Only then does it start early beside the Smagorinsky branch: its waiting blocks
+// take their places first, which puts the two inverse passes one behind the other and is
+// faster where they fill the device anyway (us a step, overlapped against not: 96^2 x 48
+// double, 1.46 waves of blocks, 321 / 349; 100^2 x 37 double 360 / 395; 24 members
+// 64^2 x 32 mixed 1208 / 1327; 256^2 x 128 mixed 3243 / 3359), and takes places from the
+// longer branch where they do not (64^2 x 64 double, 1.04 waves, 249 / 232; 64^2 x 32 double
+// 169 / 158, mixed 124 / 126; 48^2 x 24 double 137 / 132).
+bool adv_inverse_fills_device(const bld_handle* h, int nm) {
+    const Space& s = h->adv;
+    if (!s.yl) return false;
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+    const bld_yl::Shape y = bld_yl::inv_shape(s.P2, h->fp32, false);
+    const long long blocks = 6LL * nm * ((h->g.K1 + y.NL - 1) / y.NL) * h->g.n3;
+    return 4 * blocks > 5LL * y.MINB * nsm;
+}
+
 // compute_rates! (src/Processes.jl:39-62): nonlinear processes in the reference's
 // process order (advection, then SGS), each rate written once with the linear terms
-int enqueue_rates_impl(bld_handle* h, const double2* state, double2* du, int m0, int nm,
-                       const StageFuse* sf = nullptr) {
+int enqueue_rates_kernels(bld_handle* h, const double2* state, double2* du, int m0, int nm, const StageFuse* sf) {
     // With both spaces the Smagorinsky inverse and x passes run beside the advection's
     // three passes on the handle's second stream (a branch of the step graph): they share
     // only the state they read.  The Smagorinsky forward pass, which adds to the rates of
@@ -948,13 +982,20 @@ int enqueue_rates_impl(bld_handle* h, const double2* state, double2* du, int m0,
         const cudaStream_t st = h->stream;
         CUDA_TRY(cudaEventRecord(h->ev_fork, st));
         CUDA_TRY(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
+        const bool overlap = h->overlap;
         h->stream = h->side;
+        // inside the branches no other launch is overlapped: blocks that wait there would
+        // hold places the other branch can use (64^2 x 32 double: 179 us a step with all of
+        // them overlapped, 158 with none)
+        h->overlap = false;
         int rc = enqueue_inv_y(h, 1, state, m0, nm);
         if (rc == BLD_OK) rc = enqueue_x(h, 1, m0, nm);
         h->stream = st;
+        h->overlap = overlap && adv_inverse_fills_device(h, nm);
         // joined in any case: a capture must not end with a loose branch
         const cudaError_t e = cudaEventRecord(h->ev_join, h->side);
         if (rc == BLD_OK && e == cudaSuccess) rc = enqueue_inv_y(h, 0, state, m0, nm);
+        h->overlap = false;
         if (rc == BLD_OK && e == cudaSuccess) rc = enqueue_x(h, 0, m0, nm);
         if (rc == BLD_OK && e == cudaSuccess) rc = enqueue_fwd_y(h, 0, true, false, state, du, m0, nm, nullptr);
         if (e == cudaSuccess) CUDA_TRY(cudaStreamWaitEvent(st, h->ev_join, 0));
@@ -965,6 +1006,7 @@ int enqueue_rates_impl(bld_handle* h, const double2* state, double2* du, int m0,
     for (int sp = 0; sp < 2; ++sp) {
         if (!(sp == 0 ? h->adv.on : h->sgs.on)) continue;
         BLD_TRY(enqueue_inv_y(h, sp, state, m0, nm));
+        h->overlap = true;
         BLD_TRY(enqueue_x(h, sp, m0, nm));
     }
     bool first = true;
@@ -979,6 +1021,16 @@ int enqueue_rates_impl(bld_handle* h, const double2* state, double2* du, int m0,
         BLD_TRY(enqueue_linear(h, state, du, m0, nm));
     }
     return BLD_OK;
+}
+
+// A right-hand side; in line, its kernels after the first are launched overlapped, the
+// first where the caller's h->overlap says so.
+int enqueue_rates_impl(bld_handle* h, const double2* state, double2* du, int m0, int nm,
+                       const StageFuse* sf = nullptr) {
+    const bool overlap = h->overlap;
+    const int rc = enqueue_rates_kernels(h, state, du, m0, nm, sf);
+    h->overlap = overlap;
+    return rc;
 }
 
 // The stage update can ride on the last forward y pass when that pass is the
@@ -1049,8 +1101,8 @@ int enqueue_project(bld_handle* h, int kind, double dt, const double2* u, const 
         const size_t sm = project_tile_smem(n3, ln);
 #define BLD_TILE(L, N)                                                                                          \
     if (lmax == L && ln == N) {                                                                                \
-        if (kind == S_EULER) k_project_tile<L, N, true><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag); \
-        else k_project_tile<L, N><<<grid, block, sm, h->stream>>>(a, umap, gmap, h->flag);                      \
+        const auto k = kind == S_EULER ? k_project_tile<L, N, true> : k_project_tile<L, N>;                     \
+        CUDA_TRY(bld_util::launch(k, grid, block, sm, h->stream, h->overlap && overlap_on(), a, umap, gmap, h->flag)); \
     }
         BLD_TILE(8, 4)
         BLD_TILE(8, 8)
@@ -1112,65 +1164,72 @@ int enqueue_step(bld_handle* h, int method, double dt, bool ab2_first, int chain
     const int B = h->B;
     struct MaskScope {
         bld_handle* h;
-        ~MaskScope() { h->mask_on = false; }
+        ~MaskScope() { h->mask_on = h->overlap = false; }
     } scope{h};
     h->mask_on = true;
+    // every kernel but the step's first is launched overlapped (AB2 has copies between them)
+    auto project = [&](int kind, double pdt, const double2* u, const double2* t, const double2* du, const double2* dp,
+                       double2* out) {
+        const int rc = enqueue_project(h, kind, pdt, u, t, du, dp, out, 0, B);
+        h->overlap = method != BLD_AB2;
+        return rc;
+    };
     switch (method) {
         case BLD_EULER:
-            BLD_TRY(enqueue_project(h, S_EULER, dt, h->u, nullptr, h->du, nullptr, h->u, 0, B));
+            BLD_TRY(project(S_EULER, dt, h->u, nullptr, h->du, nullptr, h->u));
             BLD_TRY(enqueue_rates(h, h->u, h->du, 0, B));
             break;
         case BLD_SSPRK22:
             if (chain & CHAIN_ENTER)
-                BLD_TRY(enqueue_project(h, S_NONE, dt, h->t, nullptr, nullptr, nullptr, h->t, 0, B));
+                BLD_TRY(project(S_NONE, dt, h->t, nullptr, nullptr, nullptr, h->t));
             else
-                BLD_TRY(enqueue_project(h, S_EULER, dt, h->u, nullptr, h->du, nullptr, h->t, 0, B));
+                BLD_TRY(project(S_EULER, dt, h->u, nullptr, h->du, nullptr, h->t));
             if (stage_fusable(h)) {
                 // u <- (u + t + dt f(t)) / 2 in the forward y pass (u is read and
                 // written element by element; the pass reads t), then project u
                 const StageFuse sf{h->u, h->u, 1.0, 1.0, dt, 2.0};
                 BLD_TRY(enqueue_rates_impl(h, h->t, h->du, 0, B, &sf));
-                BLD_TRY(enqueue_project(h, S_NONE, dt, h->u, nullptr, nullptr, nullptr, h->u, 0, B));
+                BLD_TRY(project(S_NONE, dt, h->u, nullptr, nullptr, nullptr, h->u));
             } else {
                 BLD_TRY(enqueue_rates(h, h->t, h->du, 0, B));
-                BLD_TRY(enqueue_project(h, S_RK22_2, dt, h->u, h->t, h->du, nullptr, h->u, 0, B));
+                BLD_TRY(project(S_RK22_2, dt, h->u, h->t, h->du, nullptr, h->u));
             }
             BLD_TRY(enqueue_trailing_rates(h, dt, chain));
             break;
         case BLD_SSPRK33:
             if (chain & CHAIN_ENTER)
-                BLD_TRY(enqueue_project(h, S_NONE, dt, h->t, nullptr, nullptr, nullptr, h->t, 0, B));
+                BLD_TRY(project(S_NONE, dt, h->t, nullptr, nullptr, nullptr, h->t));
             else
-                BLD_TRY(enqueue_project(h, S_EULER, dt, h->u, nullptr, h->du, nullptr, h->t, 0, B));
+                BLD_TRY(project(S_EULER, dt, h->u, nullptr, h->du, nullptr, h->t));
             if (stage_fusable(h)) {
                 // second stage into du (free once the first stage consumed it; the
                 // pass reads t, so the stage value cannot overwrite t in place)
                 const StageFuse s2{h->u, h->du, 3.0, 1.0, dt, 4.0};
                 BLD_TRY(enqueue_rates_impl(h, h->t, h->du, 0, B, &s2));
-                BLD_TRY(enqueue_project(h, S_NONE, dt, h->du, nullptr, nullptr, nullptr, h->du, 0, B));
+                BLD_TRY(project(S_NONE, dt, h->du, nullptr, nullptr, nullptr, h->du));
                 // third stage into u from the second-stage state held in du; the
                 // partial rates of a first forward pass (when two physical-domain
                 // spaces contribute) go to t, which the first stage left free
                 const StageFuse s3{h->u, h->u, 1.0, 2.0, 2.0 * dt, 3.0};
                 BLD_TRY(enqueue_rates_impl(h, h->du, h->t, 0, B, &s3));
-                BLD_TRY(enqueue_project(h, S_NONE, dt, h->u, nullptr, nullptr, nullptr, h->u, 0, B));
+                BLD_TRY(project(S_NONE, dt, h->u, nullptr, nullptr, nullptr, h->u));
             } else {
                 BLD_TRY(enqueue_rates(h, h->t, h->du, 0, B));
-                BLD_TRY(enqueue_project(h, S_RK33_2, dt, h->u, h->t, h->du, nullptr, h->t, 0, B));
+                BLD_TRY(project(S_RK33_2, dt, h->u, h->t, h->du, nullptr, h->t));
                 BLD_TRY(enqueue_rates(h, h->t, h->du, 0, B));
-                BLD_TRY(enqueue_project(h, S_RK33_3, dt, h->u, h->t, h->du, nullptr, h->u, 0, B));
+                BLD_TRY(project(S_RK33_3, dt, h->u, h->t, h->du, nullptr, h->u));
             }
             BLD_TRY(enqueue_trailing_rates(h, dt, chain));
             break;
         case BLD_AB2: {
             const size_t bytes = (size_t)B * h->g.mstride * sizeof(double2);
             if (ab2_first) {
-                BLD_TRY(enqueue_project(h, S_EULER, dt, h->u, nullptr, h->du, nullptr, h->u, 0, B));
+                BLD_TRY(project(S_EULER, dt, h->u, nullptr, h->du, nullptr, h->u));
                 CUDA_TRY(cudaMemcpyAsync(h->dp, h->du, bytes, cudaMemcpyDeviceToDevice, h->stream));
                 BLD_TRY(enqueue_rates(h, h->u, h->du, 0, B));
-                BLD_TRY(enqueue_project(h, S_AB2_1, dt, h->u, nullptr, h->du, h->dp, h->u, 0, B));
+                BLD_TRY(project(S_AB2_1, dt, h->u, nullptr, h->du, h->dp, h->u));
             } else {
-                BLD_TRY(enqueue_project(h, S_AB2, dt, h->u, nullptr, h->du, h->dp, h->u, 0, B));
+                BLD_TRY(project(S_AB2, dt, h->u, nullptr, h->du, h->dp, h->u));
                 CUDA_TRY(cudaMemcpyAsync(h->dp, h->du, bytes, cudaMemcpyDeviceToDevice, h->stream));
             }
             BLD_TRY(enqueue_rates(h, h->u, h->du, 0, B));

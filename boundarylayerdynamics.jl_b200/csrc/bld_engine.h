@@ -214,6 +214,9 @@ struct bld_handle {
     std::map<std::vector<const void*>, cudaGraphExec_t> ens_graphs;  // parent graphs led by this handle
     size_t bytes = 0;
     int proj_euler = 0;          // 1: the Euler stage of a step by k_project_tile too (autotuned)
+    // kernels enqueued now may be set up while the one before them on the stream ends
+    // (overlapped launches; off for the first kernel of a schedule and after a join)
+    bool overlap = false;
     cudaStream_t side = nullptr;   // second branch of the right-hand side (with both physical spaces)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 };

@@ -90,6 +90,7 @@ struct InvYArgs {
     const double* alpha_i;       // [n3-1]
     FftPlan plan;
     const void* tw;
+    int overlap;                 // launched overlapping the kernel before it (k_inv_yl)
 };
 
 // value of spectral term `op` at (z, j, k1); D1 = i*d1, D2 = i*d2
@@ -986,6 +987,7 @@ struct FwdYArgs {
     const int* active;
     FftPlan plan;
     const void* tw;
+    int overlap;               // launched overlapping the kernel before it (k_fwd_yl)
 };
 
 // Frequency-domain Laplacian with ghost layers (src/processes/molecular_diffusion.jl:57-72,

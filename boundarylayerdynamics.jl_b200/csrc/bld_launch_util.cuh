@@ -31,4 +31,22 @@ cudaError_t opt_in(K kernel, int smem, std::atomic<int> (&done)[64]) {
     return e;
 }
 
+// launches `kernel`; with `overlap` its blocks may be set up while the last blocks of the
+// kernel before it on the stream still run (they wait in grid_wait before they read
+// anything)
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool overlap, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace bld_util

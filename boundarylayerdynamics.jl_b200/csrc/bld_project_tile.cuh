@@ -277,6 +277,7 @@ template <int LMAX, int LN, bool EULER = false>
 __global__ void __launch_bounds__(LN * 32) k_project_tile(ProjArgs a, const __grid_constant__ CUtensorMap umap,
                                                         const __grid_constant__ CUtensorMap gmap, int* flag) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    grid_wait();   // every block, whether it has work or not
     __shared__ double2 sP[32][LN];
     __shared__ double sQ[32][LN];
     // the TMA destinations start on 128-byte boundaries
@@ -320,6 +321,7 @@ template <int LMAX, int LN>
 __global__ void __launch_bounds__(LN * 32) k_project_pipe(ProjArgs a, int nm, const __grid_constant__ CUtensorMap umap,
                                                         const __grid_constant__ CUtensorMap gmap, int* flag) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    grid_wait();   // every block, whether it has work or not
     __shared__ double2 sP[32][LN];
     __shared__ double sQ[32][LN];
     unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);

@@ -21,6 +21,14 @@
 // their timeout exit with no copy missing)
 __device__ long long g_bld_wait_limit = BLD_WAIT_CYCLES;
 
+// Start of a kernel that may be launched while the one before it still runs: waits until
+// that one has completed and its writes are visible, then lets the next kernel's blocks
+// be set up behind this one's last.  Without an overlapped launch both return at once.
+__device__ __forceinline__ void grid_wait() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {

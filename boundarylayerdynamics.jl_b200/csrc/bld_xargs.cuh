@@ -43,6 +43,7 @@ struct XArgs {
     // row kernels (bld_xrows.cuh): [K1] k1 * 2pi/L1, and the device's limit of bounded waits
     const double* d1;
     const long long* wait_limit;
+    int overlap;   // launched overlapping the kernel before it (row kernels)
 };
 
 // n / d for 0 <= n < 2^16 and 1 <= d < 2^16 by one multiply-high with

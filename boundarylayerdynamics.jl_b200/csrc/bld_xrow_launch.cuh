@@ -18,8 +18,7 @@ cudaError_t launch_adv_p(const XArgs& a, int nchunks, int nm, cudaStream_t st) {
         const auto k = k_adv_row<R, s.A, s.B, s.NR, s.T, s.MINB, s.sepf>;
         const int sm = ar_smem(s.A, s.B, a.g.K1, (int)sizeof(cplx<R>), s.NR, s.sepf);
         if (const cudaError_t e = opt_in(k, sm, done); e != cudaSuccess) return e;
-        k<<<dim3((a.P2 + s.NR - 1) / s.NR, nchunks, nm), s.T, sm, st>>>(a);
-        return cudaGetLastError();
+        return bld_util::launch(k, dim3((a.P2 + s.NR - 1) / s.NR, nchunks, nm), s.T, sm, st, a.overlap != 0, a);
     }
     return cudaErrorInvalidValue;
 }
@@ -32,8 +31,7 @@ cudaError_t launch_sgs_p(const XArgs& a, int nchunks, int nm, cudaStream_t st) {
         const auto k = k_sgs_x<R, s.A, s.B, s.NR, s.T, s.MINB, s.sepf>;
         const int sm = sr_smem(s.A, s.B, a.g.K1, (int)sizeof(cplx<R>), s.NR, s.sepf);
         if (const cudaError_t e = opt_in(k, sm, done); e != cudaSuccess) return e;
-        k<<<dim3(a.P2 / s.NR, nchunks, nm), s.T, sm, st>>>(a);
-        return cudaGetLastError();
+        return bld_util::launch(k, dim3(a.P2 / s.NR, nchunks, nm), s.T, sm, st, a.overlap != 0, a);
     }
     return cudaErrorInvalidValue;
 }

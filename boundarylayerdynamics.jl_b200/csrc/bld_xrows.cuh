@@ -105,6 +105,10 @@ __global__ void __launch_bounds__(T, MINB) k_adv_row(XArgs a) {
     constexpr int LW = 32 / B;   // lines per warp in forward pass 2
     static_assert(NR % 2 == 0 && B <= 32 && T % 32 == 0, "shape");
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    C* tw = reinterpret_cast<C*>(smem_raw + 128);
+    const C* twg = reinterpret_cast<const C*>(a.tw);
+    for (int i = threadIdx.x; i < P; i += T) tw[i] = twg[(i / A) * (i % A)];   // [t][q]: W_P^(t q)
+    grid_wait();   // every block, whether it has work or not
     const int n3 = a.g.n3, k1max = a.g.k1max, K1 = a.g.K1;
     const int m = a.m0 + blockIdx.z;
     BLD_SKIP_INACTIVE(a, m);
@@ -113,7 +117,6 @@ __global__ void __launch_bounds__(T, MINB) k_adv_row(XArgs a) {
     if (z0 >= z1) return;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
     unsigned char* p = smem_raw + 128;
-    C* tw = reinterpret_cast<C*>(p);
     p += xr_al(P * csz);
     C* stage = reinterpret_cast<C*>(p);
     p += xr_al(6 * NR * K1 * csz);
@@ -140,8 +143,6 @@ __global__ void __launch_bounds__(T, MINB) k_adv_row(XArgs a) {
         fence_async_shared();
         issue(jb);
     }
-    const C* twg = reinterpret_cast<const C*>(a.tw);
-    for (int i = threadIdx.x; i < P; i += T) tw[i] = twg[(i / A) * (i % A)];   // [t][q]: W_P^(t q)
     AdvCarry<R> cy[PPT];
 #pragma unroll
     for (int i = 0; i < PPT; ++i) cy[i] = AdvCarry<R>{R(0), R(0), R(0), R(0)};
@@ -412,6 +413,10 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
     constexpr int LW = 32 / B;   // lines per warp in forward pass 2
     static_assert((NR == 1 || NR % 2 == 0) && B <= 32 && A % 2 == 0 && T % 32 == 0, "shape");
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    C* tw = reinterpret_cast<C*>(smem_raw + 128);
+    const C* twg = reinterpret_cast<const C*>(a.tw);
+    for (int i = threadIdx.x; i < P; i += T) tw[i] = twg[(i / A) * (i % A)];   // [t][q]: W_P^(t q)
+    grid_wait();   // every block, whether it has work or not
     const int n3 = a.g.n3, k1max = a.g.k1max, K1 = a.g.K1;
     const int m = a.m0 + blockIdx.z;
     BLD_SKIP_INACTIVE(a, m);
@@ -420,7 +425,6 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
     if (z0 >= z1) return;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
     unsigned char* p = smem_raw + 128;
-    C* tw = reinterpret_cast<C*>(p);
     p += xr_al(P * csz);
     R* dk = reinterpret_cast<R*>(p);
     p += xr_al(K1 * csz / 2);
@@ -452,8 +456,6 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
         fence_async_shared();
         issue(jb);   // jb <= z0 <= n3 - 1
     }
-    const C* twg = reinterpret_cast<const C*>(a.tw);
-    for (int i = threadIdx.x; i < P; i += T) tw[i] = twg[(i / A) * (i % A)];   // [t][q]: W_P^(t q)
     for (int i = threadIdx.x; i < K1; i += T) dk[i] = (R)a.d1[i];
     SgsRow<R> cy[PPT];
 #pragma unroll

@@ -17,8 +17,8 @@ cudaError_t launch_inv_p(InvYArgs a, int nm, cudaStream_t st) {
         const int sm = smem_bytes(s.A, s.B, s.NL, (int)sizeof(cplx<R>), 1);
         if (const cudaError_t e = bld_util::opt_in(k, sm, done); e != cudaSuccess) return e;
         a.NL = s.NL;
-        k<<<dim3(a.nterms * nm, (a.g.K1 + s.NL - 1) / s.NL, a.g.n3), (s.A > s.B ? s.A : s.B) * s.NL, sm, st>>>(a);
-        return cudaGetLastError();
+        return bld_util::launch(k, dim3(a.nterms * nm, (a.g.K1 + s.NL - 1) / s.NL, a.g.n3),
+                                (s.A > s.B ? s.A : s.B) * s.NL, sm, st, a.overlap != 0, a);
     }
     return cudaErrorInvalidValue;
 }
@@ -32,8 +32,8 @@ cudaError_t launch_fwd_p(FwdYArgs a, int nm, cudaStream_t st) {
         const int sm = smem_bytes(s.A, s.B, s.NL, (int)sizeof(cplx<R>), SGS ? 2 : 1);
         if (const cudaError_t e = bld_util::opt_in(k, sm, done); e != cudaSuccess) return e;
         a.NL = s.NL;
-        k<<<dim3(a.fields * nm, (a.g.K1 + s.NL - 1) / s.NL, a.g.n3), (s.A > s.B ? s.A : s.B) * s.NL, sm, st>>>(a);
-        return cudaGetLastError();
+        return bld_util::launch(k, dim3(a.fields * nm, (a.g.K1 + s.NL - 1) / s.NL, a.g.n3),
+                                (s.A > s.B ? s.A : s.B) * s.NL, sm, st, a.overlap != 0, a);
     }
     return cudaErrorInvalidValue;
 }

@@ -94,6 +94,9 @@ __global__ void __launch_bounds__((A > B ? A : B) * NL, MINB) k_inv_yl(InvYArgs 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* tw = reinterpret_cast<C*>(smem_raw);
     C* buf = tw + P;
+    const C* twg = reinterpret_cast<const C*>(a.tw);
+    for (int i = threadIdx.x; i < P; i += T) tw[i] = twg[(i / A) * (i % A)];   // [s][j]: W_P^(j s)
+    grid_wait();   // every block, whether it has work or not
     const int t = blockIdx.x % a.nterms, m = a.m0 + blockIdx.x / a.nterms;
     BLD_SKIP_INACTIVE(a, m);
     const int z = blockIdx.z;
@@ -104,8 +107,6 @@ __global__ void __launch_bounds__((A > B ? A : B) * NL, MINB) k_inv_yl(InvYArgs 
     const int l = threadIdx.x % NL, j = threadIdx.x / NL;
     const int k1 = blockIdx.y * NL + l;
     const bool ok = k1 < K1;
-    const C* twg = reinterpret_cast<const C*>(a.tw);
-    for (int i = threadIdx.x; i < P; i += T) tw[i] = twg[(i / A) * (i % A)];   // [s][j]: W_P^(j s)
     const double2* S = a.state + (long long)m * a.g.mstride;
     if (B >= A || j < B) {
         if constexpr (SGS) {
@@ -217,6 +218,11 @@ __global__ void __launch_bounds__((A > B ? A : B) * NL, MINB) k_fwd_yl(FwdYArgs 
     constexpr int P = A * B, AP = task_stride(A, NL, (int)sizeof(C)), T = (A > B ? A : B) * NL, NJ = T / NL;
     constexpr int SB = B * AP * NL;   // elements of one line set
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    C* tw = reinterpret_cast<C*>(smem_raw);
+    C* buf = tw + P;
+    const C* twg = reinterpret_cast<const C*>(a.tw);
+    for (int i = threadIdx.x; i < P; i += T) tw[i] = twg[(i / A) * (i % A)];   // [s][j]: W_P^(j s)
+    grid_wait();   // every block, whether it has work or not
     const int fi = blockIdx.x % a.fields, m = a.m0 + blockIdx.x / a.fields;
     BLD_SKIP_INACTIVE(a, m);
     const int f = a.field0 + fi;
@@ -225,10 +231,6 @@ __global__ void __launch_bounds__((A > B ? A : B) * NL, MINB) k_fwd_yl(FwdYArgs 
     const int nz = (f == 2) ? g.n3 - 1 : g.n3;
     if (z >= nz) return;
     const int K1 = g.K1;
-    C* tw = reinterpret_cast<C*>(smem_raw);
-    C* buf = tw + P;
-    const C* twg = reinterpret_cast<const C*>(a.tw);
-    for (int i = threadIdx.x; i < P; i += T) tw[i] = twg[(i / A) * (i % A)];   // [s][j]: W_P^(j s)
     const int l = threadIdx.x % NL, j = threadIdx.x / NL;
     const int k1 = blockIdx.y * NL + l;
     const bool ok = k1 < K1;

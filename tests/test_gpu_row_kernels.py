@@ -99,6 +99,41 @@ def test_members_and_mask(oracle, BLD):
         assert np.array_equal(gm.get_state(1)[f], before[f]), f
 
 
+@pytest.mark.parametrize("res,les", [((16, 16, 8), True), ((64, 64, 32), True), ((96, 96, 48), True), ((64, 48, 33), False),
+                                     ((192, 192, 24), False)])
+@pytest.mark.parametrize("method", ["SSPRK33", "SSPRK22", "Euler", "AB2"])
+def test_overlapped_launches_change_nothing(oracle, BLD, res, les, method):
+    """Step graphs whose kernels are set up while the one before them ends give the bits of
+    graphs without (the kernels and their order are the same)."""
+    import os
+    if les:
+        om = _les(oracle, res)
+        build = lambda: _les(BLD, res)
+    else:
+        dom = lambda api: api.Domain((4 * math.pi, 2 * math.pi, 2.0), api.SmoothWall(), api.SmoothWall())
+        procs = lambda api: api.incompressible_flow(1 / 180, constant_forcing=1)
+        om = oracle.Model(res, dom(oracle), procs(oracle))
+        build = lambda: BLD.Model(res, dom(BLD), procs(BLD))
+    st = _state(om, seed=31)
+    out = []
+    for off in ("0", "1"):
+        saved = os.environ.get("BLD_NO_OVERLAP")
+        os.environ["BLD_NO_OVERLAP"] = off
+        try:
+            gm = build()
+            gm.set_state(st)
+            gm.prepare()
+            gm.step(7, 1e-4, method)
+            out.append(gm.get_state())
+        finally:
+            if saved is None:
+                del os.environ["BLD_NO_OVERLAP"]
+            else:
+                os.environ["BLD_NO_OVERLAP"] = saved
+    for f in om.fields:
+        assert np.array_equal(out[0][f], out[1][f]), (res, method, f)
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_bounded_wait_timeout_exit(oracle, BLD, precision):
     """With the device's wait limit at 0 the kernels take their timeout exit and the call
