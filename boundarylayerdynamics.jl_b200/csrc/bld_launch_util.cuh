@@ -16,18 +16,24 @@ inline cudaError_t init_tables() {
     return e == cudaSuccess ? cudaMemcpyToSymbol(c_wtab32, h_wtab32, sizeof(h_wtab32)) : e;
 }
 
-// opts `kernel` in to `smem` bytes and the largest shared-memory carveout on the current
-// device, the first time and whenever more bytes are asked for
+// the most dynamic shared memory a B200 block may opt into
+constexpr int kMaxSmem = 227 * 1024;
+
+// Opts `kernel` in to kMaxSmem bytes of dynamic shared memory and the largest carveout on
+// the current device, once per device.  The limit is the same whatever `smem` the launch
+// asks for (the bytes of one instantiation depend on the grid): threads that come here at
+// the same time set the same value, so none lowers a limit another one relies on.
 template <typename K>
 cudaError_t opt_in(K kernel, int smem, std::atomic<int> (&done)[64]) {
+    if (smem > kMaxSmem) return cudaErrorInvalidValue;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev < 64 && done[dev].load() >= smem) return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (dev < 64 && done[dev].load()) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess && dev < 64) done[dev].store(smem);
+    if (e == cudaSuccess && dev < 64) done[dev].store(1);
     return e;
 }
 

@@ -1,0 +1,42 @@
+"""Host code of the native library against fakes of the CUDA runtime, without a GPU.
+
+Each program of tests/native is compiled with nvcc against the library's headers and
+linked to the shared runtime, some of whose functions its .cpp file replaces.
+"""
+
+import glob
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import PKG_DIR, REPO
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def _nvcc():
+    return shutil.which("nvcc") or (os.path.exists("/usr/local/cuda/bin/nvcc") and "/usr/local/cuda/bin/nvcc") or None
+
+
+def run_native(tmp_path, name):
+    nvcc = _nvcc()
+    if nvcc is None:
+        pytest.skip("nvcc is not installed")
+    lib = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "lib64")
+    exe = str(tmp_path / name)
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-cudart", "shared", "-Xlinker", "-rpath",
+                    "-Xlinker", lib, "-diag-suppress", "177,550,1886", "-I", os.path.join(REPO, "include"), "-I",
+                    os.path.join(PKG_DIR, "csrc"), "-o", exe, *sorted(glob.glob(os.path.join(HERE, "native", name + "*.c*"))), "-lpthread"],
+                   check=True)
+    out = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0, (out.returncode, out.stdout, out.stderr)
+    return out.stdout.split()
+
+
+def test_shared_memory_limit_never_falls(tmp_path):
+    """Two threads that opt one kernel in for two grids leave it with room for both."""
+    e0, e1, limit, larger = map(int, run_native(tmp_path, "opt_in_threads"))
+    assert (e0, e1) == (0, 0)
+    assert limit >= larger
