@@ -102,7 +102,7 @@ __device__ __forceinline__ void project_tile_body(const ProjArgs& a, double2* ti
 #pragma unroll
             for (int q = 0; q < LMAX; ++q)
                 if ((FULL || q < len) && (f < 2 || z0 + q < n - 1))
-                    D[q] = __ldg(du + (long long)(f * n + z0 + q) * F);
+                    D[q] = ld_written(du + (long long)(f * n + z0 + q) * F);
 #pragma unroll
             for (int q = 0; q < LMAX; ++q)
                 if ((FULL || q < len) && (f < 2 || z0 + q < n - 1)) {

@@ -40,8 +40,8 @@ __host__ __device__ constexpr int smem_bytes(int A, int B, int NL, int csz, int 
 // inverse pass 1 for term kind OP: gather the padded spectral line straight from the
 // state, radix-A DFT, store
 template <typename R, int A, int B, int NL, int BAND, int OP>
-__device__ __forceinline__ void inv_pass1(const InvYArgs& a, const double2* __restrict__ S, int f, int z, int k1,
-                                          bool ok, int j, cplx<R>* buf) {
+__device__ __forceinline__ void inv_pass1(const InvYArgs& a, const double2* S, int f, int z, int k1, bool ok, int j,
+                                          cplx<R>* buf) {
     using C = cplx<R>;
     constexpr int P = A * B, AP = task_stride(A, NL, (int)sizeof(C));
     const Geo& g = a.g;
@@ -285,6 +285,8 @@ __global__ void __launch_bounds__((A > B ? A : B) * NL, MINB) k_fwd_yl(FwdYArgs 
             dd1 = ok ? __ldg(a.lin.DD1 + k1) : 0.0;
         }
         if (!ok) return;
+        // the state may take the non-coherent path: it was complete before the x pass began,
+        // and this kernel is launched once that has
         const double2* S0 = MODE == 1 ? Sf + (long long)w0 * g.F + k1 : nullptr;
         const double2* Sz = MODE != 1 && FZ != 0 ? Sf + (long long)z * g.F + k1 : nullptr;
         for (int jj = j; jj < K2; jj += NJ) {

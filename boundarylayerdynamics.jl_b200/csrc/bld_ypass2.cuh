@@ -37,29 +37,29 @@ __host__ __device__ constexpr int y2_min_blocks_inv(int threads) {
 
 // spectral term `OP` of the inverse pass at mode (jj, k1) of layer z; the
 // pointers address layer z of u, v, w (Su1/Sv1: layer z + 1); same arithmetic as
-// inv_term_value (src/derivatives.jl:67-80,198-230)
+// inv_term_value (src/derivatives.jl:67-80,198-230).  k_inv_yl is launched while the
+// kernel that writes the state may still run
 template <int OP>
-__device__ __forceinline__ double2 y2_term(const double2* __restrict__ Sf, const double2* __restrict__ Su,
-                                           const double2* __restrict__ Sv, const double2* __restrict__ Sw, int F,
-                                           int mo, double e1, double e2, double al) {
+__device__ __forceinline__ double2 y2_term(const double2* Sf, const double2* Su, const double2* Sv, const double2* Sw,
+                                           int F, int mo, double e1, double e2, double al) {
     if constexpr (OP == T_DIRECT) {
-        return __ldg(Sf + mo);
+        return ld_written(Sf + mo);
     } else if constexpr (OP == T_D1) {
-        const double2 s = __ldg(Sf + mo);
+        const double2 s = ld_written(Sf + mo);
         return make_double2(-e1 * s.y, e1 * s.x);
     } else if constexpr (OP == T_D2) {
-        const double2 s = __ldg(Sf + mo);
+        const double2 s = ld_written(Sf + mo);
         return make_double2(-e2 * s.y, e2 * s.x);
     } else if constexpr (OP == T_VORT1) {  // D2 w - (-a v(z) + a v(z+1))
-        const double2 w = __ldg(Sw + mo), v0 = __ldg(Sv + mo), v1 = __ldg(Sv + F + mo);
+        const double2 w = ld_written(Sw + mo), v0 = ld_written(Sv + mo), v1 = ld_written(Sv + F + mo);
         const double dzx = -al * v0.x + al * v1.x, dzy = -al * v0.y + al * v1.y;
         return make_double2(-e2 * w.y - dzx, e2 * w.x - dzy);
     } else if constexpr (OP == T_VORT2) {  // (-a u(z) + a u(z+1)) - D1 w
-        const double2 w = __ldg(Sw + mo), u0 = __ldg(Su + mo), u1 = __ldg(Su + F + mo);
+        const double2 w = ld_written(Sw + mo), u0 = ld_written(Su + mo), u1 = ld_written(Su + F + mo);
         const double dzx = -al * u0.x + al * u1.x, dzy = -al * u0.y + al * u1.y;
         return make_double2(dzx - (-e1 * w.y), dzy - e1 * w.x);
     } else {  // T_VORT3: D1 v - D2 u
-        const double2 v = __ldg(Sv + mo), u = __ldg(Su + mo);
+        const double2 v = ld_written(Sv + mo), u = ld_written(Su + mo);
         return make_double2(-e1 * v.y - (-e2 * u.y), e1 * v.x - e2 * u.x);
     }
 }
