@@ -1792,35 +1792,59 @@ static int enqueue_profile_sample(bld_handle* h, double w) {
     return BLD_OK;
 }
 
+// one step of `method` and, while the mean profiles are on, their sample
+static int enqueue_sampled_step(bld_handle* h, int method, double dt, bool ab2_first, int chain = 0) {
+    BLD_TRY(enqueue_step(h, method, dt, ab2_first, chain));
+    if (!h->prof_on) return BLD_OK;
+    h->mask_on = true;
+    const int st = enqueue_profile_sample(h, 0.5 * dt);
+    h->mask_on = false;
+    return st;
+}
+
 // captures one step of `method` (regular steps; AB2 after its start-up step) into
-// a CUDA graph, kept as source graph and instantiated executable
-static int step_graph(bld_handle* h, int method, double dt, int chain = 0) {
+// a CUDA graph
+static int step_source(bld_handle* h, int method, double dt, int chain, cudaGraph_t* out) {
     const auto key = std::make_pair(gkey(h, method) + 32 * chain, dt);
-    if (h->graphs.count(key)) return BLD_OK;
-    cudaGraph_t graph;
-    CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    int st = enqueue_step(h, method, dt, false, chain);
-    if (st == BLD_OK && h->prof_on) {
-        h->mask_on = true;
-        st = enqueue_profile_sample(h, 0.5 * dt);
-        h->mask_on = false;
+    auto it = h->graph_src.find(key);
+    if (it == h->graph_src.end()) {
+        cudaGraph_t graph;
+        CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+        const int st = enqueue_sampled_step(h, method, dt, false, chain);
+        const cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
+        if (st != BLD_OK) {
+            if (ce == cudaSuccess) cudaGraphDestroy(graph);
+            return st;
+        }
+        CUDA_TRY(ce);
+        it = h->graph_src.emplace(key, graph).first;
     }
-    cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
-    if (st != BLD_OK) {
-        if (ce == cudaSuccess) cudaGraphDestroy(graph);
-        return st;
-    }
-    CUDA_TRY(ce);
-    cudaGraphExec_t exec;
-    cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-    if (ie != cudaSuccess) {
-        cudaGraphDestroy(graph);
-        CUDA_TRY(ie);
-    }
-    h->graphs.emplace(key, exec);
-    h->graph_src.emplace(key, graph);
+    *out = it->second;
     return BLD_OK;
 }
+
+// ... and its executable form (an ensemble's parent graph takes the source alone)
+static int step_graph(bld_handle* h, int method, double dt, int chain, cudaGraphExec_t* out) {
+    const auto key = std::make_pair(gkey(h, method) + 32 * chain, dt);
+    auto it = h->graphs.find(key);
+    if (it == h->graphs.end()) {
+        cudaGraph_t graph;
+        BLD_TRY(step_source(h, method, dt, chain, &graph));
+        cudaGraphExec_t exec;
+        CUDA_TRY(cudaGraphInstantiate(&exec, graph, 0));
+        it = h->graphs.emplace(key, exec).first;
+    }
+    *out = it->second;
+    return BLD_OK;
+}
+
+// Steps of one method and time step that are enqueued kernel by kernel before graphs are
+// made for them.  Capturing and instantiating a step with both processes takes 0.27 ms
+// (0.11 ms without the Smagorinsky branch), and a graph step is 35 (16^2 x 8) to 75 us
+// (64^2 x 32) shorter than an enqueued one, so about four steps pay for a graph; a program
+// that changes its time step from call to call never does (first step of a new model or a
+// new time step 415 -> 130 us at 16^2 x 8, 510 -> 260 us at 64^2 x 32).
+constexpr int64_t kEnqueuedSteps = 4;
 
 int32_t bld_step(bld_handle* h, int64_t nsteps, double dt, int32_t method) {
     BLD_TRY(step_impl(h, nsteps, dt, method));
@@ -1841,46 +1865,33 @@ static int step_impl(bld_handle* h, int64_t nsteps, double dt, int32_t method) {
     if (method == BLD_AB2) {
         if (h->ab2_started && h->ab2_dt != dt) return fail(BLD_ERR_ARGUMENT, "Cannot change time step for multi-step methods");
         if (!h->ab2_started) {
-            BLD_TRY(enqueue_step(h, method, dt, true));
-            if (h->prof_on) {
-                h->mask_on = true;
-                const int st = enqueue_profile_sample(h, 0.5 * dt);
-                h->mask_on = false;
-                BLD_TRY(st);
-            }
+            BLD_TRY(enqueue_sampled_step(h, method, dt, true));
             h->ab2_started = true;
             h->ab2_dt = dt;
             done = 1;
         }
     }
-    if (done < nsteps) {
-        // chained steps: the first leaves the next step's first stage value in t,
-        // the middle ones enter and leave, the last one enters and ends with f(u)
-        const bool chain = nsteps - done >= 2 && chain_ok(h, method);
-        auto graph_for = [&](int c, cudaGraphExec_t* g) -> int {
-            const auto key = std::make_pair(gkey(h, method) + 32 * c, dt);
-            auto it = h->graphs.find(key);
-            if (it == h->graphs.end()) {
-                BLD_TRY(step_graph(h, method, dt, c));
-                it = h->graphs.find(key);
-            }
-            *g = it->second;
-            return BLD_OK;
-        };
-        if (!chain) {
-            cudaGraphExec_t g;
-            BLD_TRY(graph_for(0, &g));
-            for (; done < nsteps; ++done) CUDA_TRY(cudaGraphLaunch(g, h->stream));
-        } else {
-            cudaGraphExec_t gfirst, gmid, glast;
-            BLD_TRY(graph_for(CHAIN_LEAVE, &gfirst));
-            BLD_TRY(graph_for(CHAIN_ENTER | CHAIN_LEAVE, &gmid));
-            BLD_TRY(graph_for(CHAIN_ENTER, &glast));
-            const int64_t last = nsteps - 1;
-            for (; done < nsteps; ++done)
-                CUDA_TRY(cudaGraphLaunch(done == 0 ? gfirst : (done == last ? glast : gmid), h->stream));
-        }
+    if (done == nsteps) return BLD_OK;
+    // chained steps: the first leaves the next step's first stage value in t,
+    // the middle ones enter and leave, the last one enters and ends with f(u)
+    const bool chain = nsteps - done >= 2 && chain_ok(h, method);
+    const int64_t first = done, last = nsteps - 1;
+    auto variant = [&](int64_t step) {
+        return !chain ? 0 : step == first ? CHAIN_LEAVE : step == last ? CHAIN_ENTER : CHAIN_ENTER | CHAIN_LEAVE;
+    };
+    const auto key = std::make_pair(gkey(h, method), dt);
+    if (h->enqueued_steps.size() >= 256 && !h->enqueued_steps.count(key)) h->enqueued_steps.clear();
+    int64_t& enqueued = h->enqueued_steps[key];
+    if (enqueued + (nsteps - done) <= kEnqueuedSteps) {
+        for (; done < nsteps; ++done, ++enqueued) BLD_TRY(enqueue_sampled_step(h, method, dt, false, variant(done)));
+        return BLD_OK;
     }
+    enqueued = kEnqueuedSteps;
+    // every graph that the call launches is made before the first launch
+    std::map<int, cudaGraphExec_t> graphs;
+    for (int64_t step : {first, std::min(first + 1, last), last})
+        BLD_TRY(step_graph(h, method, dt, variant(step), &graphs[variant(step)]));
+    for (; done < nsteps; ++done) CUDA_TRY(cudaGraphLaunch(graphs[variant(done)], h->stream));
     return BLD_OK;
 }
 
@@ -1917,14 +1928,14 @@ int32_t bld_ensemble_step(bld_handle* const* hs, int32_t n, int64_t nsteps, doub
             cudaGraph_t parent;
             CUDA_TRY(cudaGraphCreate(&parent, 0));
             for (int i = 0; i < n; ++i) {
-                int st = step_graph(hs[i], method, dt, c);
+                cudaGraph_t child;
+                int st = step_source(hs[i], method, dt, c, &child);
                 if (st != BLD_OK) {
                     cudaGraphDestroy(parent);
                     return st;
                 }
                 cudaGraphNode_t node;
-                cudaError_t e = cudaGraphAddChildGraphNode(
-                    &node, parent, nullptr, 0, hs[i]->graph_src.at(std::make_pair(gkey(hs[i], method) + 32 * c, dt)));
+                cudaError_t e = cudaGraphAddChildGraphNode(&node, parent, nullptr, 0, child);
                 if (e != cudaSuccess) {
                     cudaGraphDestroy(parent);
                     CUDA_TRY(e);
@@ -1944,9 +1955,9 @@ int32_t bld_ensemble_step(bld_handle* const* hs, int32_t n, int64_t nsteps, doub
         BLD_TRY(parent_for(0, &g));
         for (int64_t s = 0; s < nsteps; ++s) CUDA_TRY(cudaGraphLaunch(g, lead->stream));
     } else {
-        cudaGraphExec_t gfirst, gmid, glast;
+        cudaGraphExec_t gfirst, gmid = nullptr, glast;
         BLD_TRY(parent_for(CHAIN_LEAVE, &gfirst));
-        BLD_TRY(parent_for(CHAIN_ENTER | CHAIN_LEAVE, &gmid));
+        if (nsteps > 2) BLD_TRY(parent_for(CHAIN_ENTER | CHAIN_LEAVE, &gmid));
         BLD_TRY(parent_for(CHAIN_ENTER, &glast));
         for (int64_t s = 0; s < nsteps; ++s)
             CUDA_TRY(cudaGraphLaunch(s == 0 ? gfirst : (s == nsteps - 1 ? glast : gmid), lead->stream));
@@ -2183,11 +2194,12 @@ int32_t bld_describe(bld_handle* h, char* buf, size_t len) {
     else
         snprintf(tmp, sizeof tmp, "%s\"projection\": \"k_project\"", out.size() > 1 ? ", " : "");
     out += tmp;
-    if (h->proj_tile)
-        snprintf(tmp, sizeof tmp, ", \"projection_stored\": \"%s<%d, %d>\"}",
+    if (h->proj_tile) {
+        snprintf(tmp, sizeof tmp, ", \"projection_stored\": \"%s<%d, %d>\"",
                  h->proj_pipe ? "k_project_pipe" : "k_project_tile", h->g.n3 <= 128 ? 8 : 16, h->proj_tile);
-    else
-        snprintf(tmp, sizeof tmp, "}");
+        out += tmp;
+    }
+    snprintf(tmp, sizeof tmp, ", \"step_graphs\": %zu}", h->graphs.size() + h->ens_graphs.size());
     out += tmp;
     if (out.size() + 1 > len) return fail(BLD_ERR_ARGUMENT, "buffer too small (%zu bytes needed)", out.size() + 1);
     memcpy(buf, out.c_str(), out.size() + 1);

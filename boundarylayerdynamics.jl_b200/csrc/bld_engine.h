@@ -211,6 +211,7 @@ struct bld_handle {
     double ab2_dt = 0;
     std::map<std::pair<int, double>, cudaGraphExec_t> graphs;
     std::map<std::pair<int, double>, cudaGraph_t> graph_src;   // kept for ensemble parent graphs
+    std::map<std::pair<int, double>, int64_t> enqueued_steps;  // steps that ran without a graph, per method and dt
     std::map<std::vector<const void*>, cudaGraphExec_t> ens_graphs;  // parent graphs led by this handle
     size_t bytes = 0;
     int proj_euler = 0;          // 1: the Euler stage of a step by k_project_tile too (autotuned)

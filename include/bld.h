@@ -222,7 +222,8 @@ int32_t bld_get_diverged(bld_handle* h, int32_t* out);
 
 /* The kernel variants the autotuner chose for this handle, as a JSON object
    (per physical-domain space: sizes, y-pass and x-pass kernels; the projection
-   kernel), NUL-terminated in `buf`.  Diagnostics; no reference counterpart. */
+   kernel) with the number of executable step graphs made so far, NUL-terminated in
+   `buf`.  Diagnostics; no reference counterpart. */
 int32_t bld_describe(bld_handle* h, char* buf, size_t len);
 
 /* Advances several handles on one device (e.g. the size classes of an uneven
