@@ -610,11 +610,15 @@ __device__ __forceinline__ void twopass_inplace(cplx<R>* buf, int nlines, int LP
 }
 
 // Values the Smagorinsky x pass carries from one layer to the next at one
-// (x, y) point: the previous C layer's velocities, strain and |S|^2 terms, and
-// the previous I layer's S13, S23, tau13, tau23, tau33.
+// (x, y) point: the previous C layer's velocities and strain, the previous I
+// layer's S13, S23 and eddy viscosity, and the tau33 of the C layer before.
+// |S|^2 and tau13, tau23 are formed again from these: with them kept as well, four
+// points a thread in double precision do not fit 255 registers and spill 268 bytes
+// (432^2 x 24 1100 against 945 us a pass, 480^2 x 24 1117 / 1000, and three points at
+// 384^2 x 24 577 / 556).
 template <typename R>
 struct SgsCarry {
-    R u, v, w, w1, w2, s11, s22, s33, s12, sc, s13, s23, t13, t23, t33;
+    R u, v, w, w1, w2, s11, s22, s33, s12, s13, s23, ev, t33;
 };
 
 // The Smagorinsky model at one (x, y) point of the x pass when C layer j enters
@@ -630,7 +634,7 @@ __device__ __forceinline__ void sgs_point(const XArgs& a, int j, int n3, bool ha
                                           R u1, R u2, R v1, R v2, R w, R w1, R w2, SgsCarry<R>& cy, R (&o)[8]) {
     const int c = j - 1;
     // (a) strain on C layer j (vel3_3 by dx3_i2c with Dirichlet w, :202-216)
-    R s11 = 0, s22 = 0, s33 = 0, s12 = 0, sc = 0;
+    R s11 = 0, s22 = 0, s33 = 0, s12 = 0;
     if (hasC) {
         const R ac = (R)a.alpha_c[j];
         const R wb = (j == 0) ? wlo : cy.w;
@@ -638,10 +642,9 @@ __device__ __forceinline__ void sgs_point(const XArgs& a, int j, int n3, bool ha
         s11 = u1;
         s22 = v2;
         s12 = (u2 + v1) / R(2);
-        sc = s11 * s11 + s22 * s22 + s33 * s33 + R(2) * (s12 * s12);
     }
     // (b) I layer j-1: S13, S23, eddy viscosity, tau13, tau23
-    R s13 = 0, s23 = 0, sg13 = 0, sg23 = 0;
+    R s13 = 0, s23 = 0, evi = 0;
     if (j >= 1 && j <= n3 - 1) {
         const R ai = (R)a.alpha_i[j - 1];
         s13 = ((-ai * cy.u + ai * u) + cy.w1) / R(2);
@@ -653,16 +656,15 @@ __device__ __forceinline__ void sgs_point(const XArgs& a, int j, int n3, bool ha
         t = cy.s33 + s33; si += t * t / R(4);
         t = cy.s12 + s12; si += R(2) * (t * t) / R(4);
         const R l2 = (R)lim[j - 1];
-        const R evi = sqrt(R(2) * si) * l2;
-        sg13 = R(-2) * evi * s13;
-        sg23 = R(-2) * evi * s23;
+        evi = sqrt(R(2) * si) * l2;
     }
+    const R sg13 = R(-2) * evi * s13, sg23 = R(-2) * evi * s23;
 #pragma unroll
     for (int q = 0; q < 8; ++q) o[q] = 0;
     R sg33 = 0;
     if (j >= 1) {
         // (c) C layer c = j-1
-        R scc = cy.sc;
+        R scc = cy.s11 * cy.s11 + cy.s22 * cy.s22 + cy.s33 * cy.s33 + R(2) * (cy.s12 * cy.s12);
         // S13 (:232-233); dynamic values are not interpolated (:245-249)
         if (c == 0) {
             if (a.dyn_lo) { const R d = cy.u * fs_lo; scc += R(2) * (d * d); }
@@ -693,8 +695,8 @@ __device__ __forceinline__ void sgs_point(const XArgs& a, int j, int n3, bool ha
         const R b23lo = a.dyn_lo ? ft_lo * cy.v * uh : R(0);
         const R b13hi = a.dyn_hi ? ft_hi * cy.u * uh : R(0);
         const R b23hi = a.dyn_hi ? ft_hi * cy.v * uh : R(0);
-        const R below13 = (c == 0) ? b13lo : cy.t13;
-        const R below23 = (c == 0) ? b23lo : cy.t23;
+        const R below13 = (c == 0) ? b13lo : R(-2) * cy.ev * cy.s13;
+        const R below23 = (c == 0) ? b23lo : R(-2) * cy.ev * cy.s23;
         const R above13 = (c == n3 - 1) ? b13hi : sg13;
         const R above23 = (c == n3 - 1) ? b23hi : sg23;
         const R ac = (R)a.alpha_c[c];
@@ -711,12 +713,11 @@ __device__ __forceinline__ void sgs_point(const XArgs& a, int j, int n3, bool ha
     if (j >= 1 && j <= n3 - 1) {
         cy.s13 = s13;
         cy.s23 = s23;
-        cy.t13 = sg13;
-        cy.t23 = sg23;
+        cy.ev = evi;
     }
     if (j >= 1) cy.t33 = sg33;
     if (hasC) {
-        cy.s11 = s11; cy.s22 = s22; cy.s33 = s33; cy.s12 = s12; cy.sc = sc;
+        cy.s11 = s11; cy.s22 = s22; cy.s33 = s33; cy.s12 = s12;
         cy.u = u; cy.v = v; cy.w = w; cy.w1 = w1; cy.w2 = w2;
     }
 }

@@ -1,4 +1,5 @@
-"""Host code of the native library against fakes of the CUDA runtime, without a GPU.
+"""Host code of the native library against fakes of the CUDA runtime, and what the
+compiler says of its kernels, without a GPU.
 
 Each program of tests/native is compiled with nvcc against the library's headers and
 linked to the shared runtime, some of whose functions its .cpp file replaces.
@@ -6,6 +7,7 @@ linked to the shared runtime, some of whose functions its .cpp file replaces.
 
 import glob
 import os
+import re
 import shutil
 import subprocess
 
@@ -20,16 +22,19 @@ def _nvcc():
     return shutil.which("nvcc") or (os.path.exists("/usr/local/cuda/bin/nvcc") and "/usr/local/cuda/bin/nvcc") or None
 
 
+def _flags(nvcc):
+    return [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-diag-suppress", "177,550,1886",
+            "-I", os.path.join(REPO, "include"), "-I", os.path.join(PKG_DIR, "csrc")]
+
+
 def run_native(tmp_path, name):
     nvcc = _nvcc()
     if nvcc is None:
         pytest.skip("nvcc is not installed")
     lib = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "lib64")
     exe = str(tmp_path / name)
-    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-cudart", "shared", "-Xlinker", "-rpath",
-                    "-Xlinker", lib, "-diag-suppress", "177,550,1886", "-I", os.path.join(REPO, "include"), "-I",
-                    os.path.join(PKG_DIR, "csrc"), "-o", exe, *sorted(glob.glob(os.path.join(HERE, "native", name + "*.c*"))), "-lpthread"],
-                   check=True)
+    subprocess.run([*_flags(nvcc), "-cudart", "shared", "-Xlinker", "-rpath", "-Xlinker", lib, "-o", exe,
+                    *sorted(glob.glob(os.path.join(HERE, "native", name + "*.c*"))), "-lpthread"], check=True)
     out = subprocess.run([exe], capture_output=True, text=True, timeout=60)
     assert out.returncode == 0, (out.returncode, out.stdout, out.stderr)
     return out.stdout.split()
@@ -40,3 +45,15 @@ def test_shared_memory_limit_never_falls(tmp_path):
     e0, e1, limit, larger = map(int, run_native(tmp_path, "opt_in_threads"))
     assert (e0, e1) == (0, 0)
     assert limit >= larger
+
+
+def test_sgs_block_kernels_do_not_spill(tmp_path):
+    """The values that the block Smagorinsky kernels carry from layer to layer fit their
+    registers in double precision (three and four points a thread)."""
+    nvcc = _nvcc()
+    if nvcc is None:
+        pytest.skip("nvcc is not installed")
+    out = subprocess.run([*_flags(nvcc), "-O3", "-lineinfo", "-Xptxas", "-v", "-c", "-o", str(tmp_path / "k.o"),
+                          os.path.join(HERE, "native", "sgs_block_registers.cu")], check=True, capture_output=True, text=True)
+    spills = re.findall(r"k_sgs_x\w*\n\s*\d+ bytes stack frame, (\d+) bytes spill stores", out.stderr)
+    assert spills == ["0"] * 3, out.stderr
