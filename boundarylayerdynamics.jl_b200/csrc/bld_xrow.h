@@ -21,19 +21,30 @@ constexpr bool codelet(int n) {
 }
 
 // A (a multiple of 3 for advection with the 3/2 rule, even for the Smagorinsky model)
-// times B with the smallest larger radix (registers); among equals the larger B in
-// single and the larger A in double precision (128 points: 8 x 16 against 16 x 8,
-// single 47 against 52 us, double 86 against 78 us at 128^2 x 64)
-constexpr void factor(Shape& s, int P, bool fp32, int multiple) {
+// times B with the smallest larger radix (registers).  Among equals: the larger B in
+// single precision, and in double precision for advection where it fills the lanes of
+// the last forward pass (128 points, double, 8 x 16 against 16 x 8: advection 211 / 228 us
+// at 84^2 x 512), else the larger A (Smagorinsky 86 / 78 us at 128^2 x 64).  A warp has
+// 32 / B lines in that pass; where that B leaves lanes idle, B = 16 takes its place if the
+// larger radix grows by no more than a third (us, before against now: advection 144
+// points single 164 / 117 at 96^2 x 512; Smagorinsky single 96 points 197 / 170, 288
+// 238 / 204, 384 284 / 263; double 160 points 274 / 253, 192 261 / 262, 224 283 / 236).
+constexpr void factor(Shape& s, int P, bool fp32, bool adv, int multiple) {
     int best = 1 << 30;
     for (int b = 2; b <= 32; ++b) {
         if (P % b || !codelet(b) || !codelet(P / b) || (P / b) % multiple) continue;
         const int a = P / b, larger = a > b ? a : b;
-        if (larger < best || (larger == best && fp32)) {
+        if (larger < best || (larger == best && (fp32 || (adv && 32 % b == 0)))) {
             best = larger;
             s.A = a;
             s.B = b;
         }
+    }
+    if (!s.A || 32 % s.B == 0 || P % 16) return;
+    const int a = P / 16, larger = a > 16 ? a : 16;
+    if (codelet(a) && a % multiple == 0 && 3 * larger <= 4 * best) {
+        s.A = a;
+        s.B = 16;
     }
 }
 
@@ -41,17 +52,18 @@ constexpr void factor(Shape& s, int P, bool fp32, int multiple) {
 // others (288 points, double: 96 / 128 / 192 threads 0.195 / 0.181 / 0.237 ms at
 // 192^2 x 96, single 0.099 / 0.105 / 0.114 ms).  Four rows per block up to 216 points in
 // single precision (two against four rows: 96 points 103 / 89 us at 64^2 x 768, 144 points
-// 136 / 117 us at 96^2 x 512), two elsewhere (registers, shared memory).  Blocks per SM:
-// the most whose register cap does not spill.  384 points and above in double precision
-// share the line buffer between both directions, for three blocks per SM (0.234 against
-// 0.244 ms with two at 256^2 x 64).
+// 136 / 117 us at 96^2 x 512), two elsewhere (registers, shared memory) but for radices up
+// to 8 in double precision where no third of the spectrum is empty: there every task has
+// all its inputs, and two rows leave half of the threads without one (64 points 100 / 72 us
+// at 42^2 x 768, k_adv_x2 84; with the empty third four rows are slower on a grid that does
+// not fill the chip: 96 points 14.6 / 16.7 us at 64^2 x 32).  Blocks per SM: the most whose
+// register cap does not spill (256 points, single, six / five blocks: 123 / 115 us at
+// 168^2 x 128).  384 points and above in double precision share the line buffer between
+// both directions, for three blocks per SM (0.234 against 0.244 ms with two at 256^2 x 64).
 constexpr Shape adv_shape(int P, bool fp32) {
     Shape s;
     if (P < 12 || P > (fp32 ? 768 : 432) || P == 512) return s;   // 512: no faster than k_adv_x2
-    factor(s, P, fp32, P % 3 == 0 ? 3 : 1);
-    if (P == 144) s.A = 9, s.B = 16;
-    if (P == 288) s.A = 18, s.B = 16;
-    if (P == 384) s.A = 24, s.B = 16;
+    factor(s, P, fp32, true, P % 3 == 0 ? 3 : 1);
     if (!s.A) return s;
     const int larger = s.A > s.B ? s.A : s.B;
     if (P <= 48) {
@@ -63,8 +75,9 @@ constexpr Shape adv_shape(int P, bool fp32) {
         s.MINB = s.T == 96 ? 7 : (s.T == 128 ? 5 : 4);
     } else if (fp32) {
         s.T = larger > 24 ? 192 : 96;
-        s.MINB = larger > 24 ? 2 : (larger >= 18 ? 5 : 6);
+        s.MINB = larger > 24 ? 2 : 5;
     } else {
+        s.NR = P % 3 && larger <= 8 ? 4 : 2;
         s.T = P > 216 && P < 384 ? 128 : 96;
         s.MINB = s.T == 128 || P >= 384 ? 3 : (larger <= 9 || P <= 144 ? 5 : 4);
         s.sepf = P < 384;
@@ -75,20 +88,32 @@ constexpr Shape adv_shape(int P, bool fp32) {
 // Smagorinsky (P1 = 2 k1max + 2).  Single precision: two rows per block, one above 288
 // points, and one thread per task of the last forward pass (four lines a row of B tasks:
 // 64 points 64 / 96 / 128 threads 111 / 138 / 130 us at 64^2 x 768; 256 points, one row and
-// 64 threads 280, two rows and 128 threads 240 us at 256^2 x 128).  Double precision, whose
-// carried values take 26 registers a point: one row above 144 points.
+// 64 threads 280, two rows and 128 threads 240 us at 256^2 x 128), but with one row at least
+// 96 for the wide first radices (360 points, 24 x 15: 64 / 96 threads 318 / 278 us at
+// 360^2 x 48).  Blocks per SM of 128 threads as the registers of the first radix allow
+// where every lane works and the lines are long enough to fill them (8 x 16, 128^2 x 256,
+// five / four blocks 148 / 158 us, 10 x 16 225 / 214, 18 x 16 four / three 221 / 204; but
+// 6 x 16, 96^2 x 48, five / four 31 / 29, eight of them 150 / 139), four where some lanes idle
+// (8 x 14, ten 112^2 x 16, five / four 93 / 84, 18 x 15, two 270^2 x 16, four / three
+// 98 / 128); with one row the most that do not spill
+// (five / four / three blocks at 324 points 305 / 286 / 285 us, 384 321 / 262 / 263, 432
+// 529 / 401 / 412, 480 490 / 407 / 358).
+// Double precision, whose carried values take 26 registers a point: one row above 144
+// points.
 constexpr Shape sgs_shape(int P, bool fp32) {
     Shape s;
     if (P < 12 || P > (fp32 ? 512 : 324)) return s;
-    factor(s, P, fp32, 2);
-    if (P == 96 && fp32) s.A = 6, s.B = 16;
+    factor(s, P, fp32, false, 2);
     if (!s.A) return s;
     const int larger = s.A > s.B ? s.A : s.B;
     if (fp32) {
         s.NR = P <= 288 || P % 4 ? 2 : 1;
         s.T = (4 * s.NR * s.B + 31) / 32 * 32;
         if (s.T > 160) s.T = 160;
-        s.MINB = s.T == 32 ? 16 : (s.T == 64 ? 8 : (s.T == 96 ? 5 : (s.T == 160 || s.NR == 1 ? 3 : (P == 128 ? 5 : 4))));
+        if (s.NR == 1 && s.T < 96) s.T = 96;
+        s.MINB = s.T == 32 ? 16 : (s.T == 64 ? 8 : (s.T == 96 ? 5 : 3));
+        if (s.T == 128) s.MINB = 32 % s.B || P < 128 ? 4 : (s.A <= 8 ? 5 : (s.A <= 16 ? 4 : 3));
+        if (s.NR == 1) s.MINB = larger <= 24 ? 4 : 3;
     } else {
         s.NR = P <= 144 ? 2 : 1;
         s.T = P <= 72 ? 64 : 96;

@@ -57,3 +57,24 @@ def test_sgs_block_kernels_do_not_spill(tmp_path):
                           os.path.join(HERE, "native", "sgs_block_registers.cu")], check=True, capture_output=True, text=True)
     spills = re.findall(r"k_sgs_x\w*\n\s*\d+ bytes stack frame, (\d+) bytes spill stores", out.stderr)
     assert spills == ["0"] * 3, out.stderr
+
+
+def test_row_kernel_radices(tmp_path):
+    """The radices of the in-place x kernels follow from the lanes they use: a second radix
+    that leaves lanes of a warp idle has no alternative of 16 that the rule allows, and the
+    larger radix is within a third of the smallest there is.  The blocks per SM ask for no
+    more registers than there are."""
+    codelets = (2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16, 18, 24, 32)
+    shapes = [line.split(",") for line in run_native(tmp_path, "row_shapes")]
+    assert len(shapes) > 120
+    for kind, *numbers in shapes:
+        points, fp32, a, b, rows, threads, blocks = map(int, numbers)
+        multiple = 2 if kind == "sgs" else 3 if points % 3 == 0 else 1
+        pairs = [(points // q, q) for q in codelets
+                 if points % q == 0 and points // q in codelets and points // q % multiple == 0]
+        smallest = min(map(max, pairs))
+        assert (a, b) in pairs and 3 * max(a, b) <= 4 * smallest, (kind, points, fp32, a, b)
+        if 32 % b:
+            assert all(q != 16 or 3 * max(p, q) > 4 * smallest for p, q in pairs), (kind, points, fp32, a, b)
+        # as many registers as radix-a or radix-b values take (2 or 4 each) have to remain
+        assert 65536 // (threads * blocks) >= max(a, b) * (2 if fp32 else 4), (kind, points, fp32, threads, blocks)
