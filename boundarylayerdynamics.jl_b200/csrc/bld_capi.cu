@@ -291,6 +291,10 @@ int enqueue_x_R(bld_handle* h, int sp, int m0, int nm) {
     xa.d1 = h->d1;
     xa.wait_limit = h->wait_limit;
     xa.overlap = h->overlap && overlap_on();
+    xa.d3_scale = h->d3_scale;
+    xa.d3_scale32 = (float)h->d3_scale;
+    xa.d3_alpha_c = h->d3_alpha_c;
+    xa.d3_alpha_i = h->d3_alpha_i;
     if (s.xrow) return launch_row(h, s, xa, nm);
     if (sp == 0) {
         return launch_adv_family<R>(h, s, xa, nm);
@@ -349,7 +353,10 @@ int enqueue_fwd_y_R(bld_handle* h, int sp, bool first, bool last, const double2*
     fa.lin = h->lin;
     fa.d1 = h->d1;
     fa.d2 = h->d2;
-    fa.inv_n = 1.0 / ((double)s.P1 * (double)s.P2);
+    const double inv_n = 1.0 / ((double)s.P1 * (double)s.P2);
+    // the in-place Smagorinsky kernel's sums go out times 2 d3_scale, its stresses times 2
+    fa.inv_a = sp == 1 && s.xrow ? 0.5 * inv_n / h->d3_scale : inv_n;
+    fa.inv_b = sp == 1 && s.xrow ? 0.5 * inv_n : inv_n;
     fa.flag = h->flag;
     fa.fields = 3;
     fa.field0 = 0;
@@ -1435,7 +1442,7 @@ void free_handle(bld_handle* h) {
     for (auto& kv : h->ens_graphs) cudaGraphExecDestroy(kv.second);
     void* ptrs[] = {h->u, h->t, h->du, h->dp, h->io, h->io2, h->pscr, h->gamma, h->d1, h->d2, h->DD1, h->DD2,
                     h->alpha_c, h->inv_alpha_c, h->alpha_i, h->alpha_ext, h->mean_w, h->lc2, h->li2, h->wall, h->src,
-                    h->mean_val, h->flag, h->active, h->adv.min, h->adv.mout, h->sgs.min, h->sgs.mout, h->pd_buf, h->pd_mixed,
+                    h->d3_alpha_c, h->d3_alpha_i, h->mean_val, h->flag, h->active, h->adv.min, h->adv.mout, h->sgs.min, h->sgs.mout, h->pd_buf, h->pd_mixed,
                     h->prog_small, h->prog_buf, h->prog_mixed};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -1573,6 +1580,17 @@ int32_t bld_create(const bld_config* cfg, bld_handle** out) {
     H_TRY(upload(h, &h->alpha_c, ac));
     H_TRY(upload(h, &h->inv_alpha_c, iac));
     H_TRY(upload(h, &h->alpha_i, ai));
+    if (cfg->sgs) {
+        // vertical derivatives of stresses in the in-place Smagorinsky kernel: the power of two
+        // next to 1 / (largest x wavenumber), within what single precision holds
+        if (g.k1max > 0)
+            h->d3_scale = std::exp2(std::min(60.0, std::max(-60.0, -std::round(std::log2(2.0 * M_PI / cfg->l1 * g.k1max)))));
+        std::vector<double> sc(ac), si(ai);
+        for (double& v : sc) v *= h->d3_scale;
+        for (double& v : si) v *= h->d3_scale;
+        H_TRY(upload(h, &h->d3_alpha_c, sc));
+        H_TRY(upload(h, &h->d3_alpha_i, si));
+    }
     H_TRY(upload(h, &h->alpha_ext, aext));
     H_TRY(upload(h, &h->mean_w, mw));
 
@@ -2260,7 +2278,7 @@ static int set_field_from_pd(bld_handle* h, int m, int field) {
     fa.check = 0;
     fa.du = h->u + (size_t)m * g.mstride;
     fa.du_mstride = 0;
-    fa.inv_n = 1.0 / ((double)P1 * (double)P2);
+    fa.inv_a = 1.0 / ((double)P1 * (double)P2);
     fa.flag = h->flag;
     fa.fields = 1;
     fa.field0 = field;

@@ -205,6 +205,8 @@ struct bld_handle {
     // host-side copies used by launches
     double w_lo = 0, w_hi = 0;
     int dyn_lo = 0, dyn_hi = 0;
+    double d3_scale = 1.0;                                        // XArgs::d3_scale and its tables
+    double *d3_alpha_c = nullptr, *d3_alpha_i = nullptr;
     Linear lin{};
     bool slope_valid = false;
     bool ab2_started = false;

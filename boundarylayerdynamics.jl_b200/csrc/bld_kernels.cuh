@@ -979,7 +979,9 @@ struct FwdYArgs {
     Linear lin;
     const double* d1;
     const double* d2;
-    double inv_n;              // 1/(P1*P2)
+    // factors of the transformed lines, 1/(P1 P2) times what the x pass left out: of the
+    // contributions with prefactor 1 or D1, and of the one under D2
+    double inv_a, inv_b;
     int* flag;                 // per member
     int fields;                // number of target fields (3 for rates, 1 for transforms)
     int field0;                // first target field
@@ -1181,11 +1183,11 @@ __device__ __forceinline__ void fwd_y_epilogue(const FwdYArgs& a, const cplx<R>*
                 if (o >= nout || k1 >= K1) continue;
                 const int pos = swz<C, RAD>((j <= k2max) ? j : P2 - (K2 - j));
                 const C X = res[pos * LS + l];
-                double vx = (double)X.x * a.inv_n, vy = (double)X.y * a.inv_n;
+                double vx = (double)X.x * a.inv_a, vy = (double)X.y * a.inv_a;
                 if (hasB) {
                     const C Y = res[pos * LS + NL + l];
                     const double d = a.d2[j];
-                    const double bx = (double)Y.x * a.inv_n, by = (double)Y.y * a.inv_n;
+                    const double bx = (double)Y.x * a.inv_b, by = (double)Y.y * a.inv_b;
                     vx += -d * by;
                     vy += d * bx;
                 }
@@ -1504,11 +1506,11 @@ __global__ void __launch_bounds__(384) k_fwd_y_all(FwdYArgs a) {
             if (o >= nout || k1 >= K1 || z >= nz) continue;
             const int pos = (j <= k2max) ? j : P2 - (K2 - j);
             const C X = buf[pos * NLT + f * NLF + l];
-            double vx = (double)X.x * a.inv_n, vy = (double)X.y * a.inv_n;
+            double vx = (double)X.x * a.inv_a, vy = (double)X.y * a.inv_a;
             if (hasB) {
                 const C Y = buf[pos * NLT + f * NLF + NL + l];
                 const double d = a.d2[j];
-                const double bx = (double)Y.x * a.inv_n, by = (double)Y.y * a.inv_n;
+                const double bx = (double)Y.x * a.inv_b, by = (double)Y.y * a.inv_b;
                 vx += -d * by;
                 vy += d * bx;
             }

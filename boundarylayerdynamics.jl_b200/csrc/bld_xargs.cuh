@@ -44,6 +44,12 @@ struct XArgs {
     const double* d1;
     const long long* wait_limit;
     int overlap;   // launched overlapping the kernel before it (row kernels)
+    // Smagorinsky row kernel: the power of two that a vertical stress derivative is scaled
+    // by while it shares a complex line with a stress, and alpha_c, alpha_i times it
+    double d3_scale;
+    float d3_scale32;
+    const double* d3_alpha_c;
+    const double* d3_alpha_i;
 };
 
 // n / d for 0 <= n < 2^16 and 1 <= d < 2^16 by one multiply-high with

@@ -297,6 +297,16 @@ __global__ void __launch_bounds__(T, MINB) k_adv_row(XArgs a) {
 // come in (six mixed terms: u, v, w, u_2, v_2, w_2) and per velocity component only
 // d1 tau_i1 + d3 tau_i3 and tau_i2 go out (six: the three sums, then tau12, tau22,
 // tau23).
+//
+// d3 tau_i3 shares a line with tau_i1, so both are rounded at the size of the larger, and
+// tau_i1 is multiplied by its wavenumber afterwards.  Near a wall d3 tau exceeds the
+// stresses by the vertical resolution; scaled by a power of two next to one over the
+// largest wavenumber on its way through the transform it adds nothing to the rounding of
+// d1 tau_i1 (vel1 of a right-hand side at 128^2 x 64, error against 64 bits relative to
+// separate lines: 1.077 without the scale and 1.000 with it in double, 1.074 and 1.000 in
+// single precision; 64^2 x 64 stretched, single, 1.191 and 1.000; scales from an eighth to
+// four times this one are as good).  The sums go out times 2 d3_scale, the stresses times 2
+// (the halves of the two-lines-in-one unpacking), and the forward y pass takes that back.
 __host__ __device__ constexpr int sr_lines_in(int NR) { return 4 * NR + (NR + 1) / 2; }
 // dynamic shared memory: barrier, twiddles, x wavenumbers, 6 terms x NR rows, lines
 __host__ __device__ constexpr int sr_smem(int A, int B, int K1, int csz, int NR, bool sepf) {
@@ -315,13 +325,14 @@ struct SgsRow {
 // layer-dependent factors of one step of the z walk (uniform over the block)
 template <typename R>
 struct SgsLayer {
-    R ac_j, ai_b, li_b, lc_c, ac_c, ai_c;   // alpha_c[j], alpha_i[j-1], li[j-1], lc[j-1], alpha_c[j-1], alpha_i[j-2]
+    R ac_j, ai_b, li_b, lc_c;   // alpha_c[j], alpha_i[j-1], li[j-1], lc[j-1]
+    R ac_c, ai_c;               // d3_alpha_c[j-1], d3_alpha_i[j-2]
 };
 
 // The Smagorinsky model at one point when C layer j enters, as sgs_point
 // (src/processes/static_smagorinsky.jl:129-249), with the three stresses of the I
 // nodes and d3 tau33 all given on I layer j - 2: o = (tau11, d3 tau13, tau12,
-// d3 tau23, tau13, d3 tau33, tau22, tau23).
+// d3 tau23, tau13, d3 tau33, tau22, tau23), the d3 terms times d3_scale.
 template <typename R>
 __device__ __forceinline__ void sgs_row_point(const XArgs& a, const SgsLayer<R>& y, int j, int n3, bool hasC, R fs_lo,
                                               R fs_hi, R ft_lo, R ft_hi, R wlo, R u, R v, R u1, R u2, R v1, R v2, R w,
@@ -440,6 +451,7 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
     const R fs_lo = (R)a.wall[4 * m + 0], fs_hi = (R)a.wall[4 * m + 1];
     const R ft_lo = (R)a.wall[4 * m + 2], ft_hi = (R)a.wall[4 * m + 3];
     const R wlo = (R)a.w_lo, whi = (R)a.w_hi;
+    const R d3_scale = sizeof(R) == 4 ? (R)a.d3_scale32 : (R)a.d3_scale;
     const unsigned row_bytes = (unsigned)(NR * K1 * csz);
     const long long wait_limit = *a.wait_limit;
     // staged slots: u, v, u_2, v_2 (C); w, w_2 (I, below the top layer) = mixed terms 0, 1, 3, 4, 2, 5
@@ -526,8 +538,8 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
         ly.ai_b = (j >= 1 && hasC) ? (R)__ldg(a.alpha_i + j - 1) : R(0);
         ly.li_b = (j >= 1 && hasC) ? (R)lim[j - 1] : R(0);
         ly.lc_c = j >= 1 ? (R)lcm[j - 1] : R(0);
-        ly.ac_c = j >= 1 ? (R)__ldg(a.alpha_c + j - 1) : R(0);
-        ly.ai_c = j >= 2 ? (R)__ldg(a.alpha_i + j - 2) : R(0);
+        ly.ac_c = j >= 1 ? (R)__ldg(a.d3_alpha_c + j - 1) : R(0);
+        ly.ai_c = j >= 2 ? (R)__ldg(a.d3_alpha_i + j - 2) : R(0);
         // ---- the model at one point of one row
 #pragma unroll
         for (int i = 0; i < PPT; ++i) {
@@ -578,7 +590,8 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
             for (int t = 0; t < A; ++t) x[t] = src[t * BS];
             dft<R, A, -1>(x);
             const int partner = ok && kp ? lane + B - 2 * kp : lane;
-            // first result: d1 tau + d3 tau of lines 0..2, tau22 of line 3; second: tau12, tau23
+            // first result: d1 tau + d3 tau of lines 0..2 (times 2 d3_scale), tau22 of line 3;
+            // second: tau12, tau23 (all times 2)
             const bool first = ok && (q == 2 ? doI : doC), second = ok && (q == 1 ? doC : q == 3 && doI);
             C* o1 = mrow_w(Mout, a, q < 3 ? q : 4, q == 2 ? j - 2 : c, y0 + r) + kp;
             C* o2 = mrow_w(Mout, a, q == 1 ? 3 : 5, q == 1 ? c : j - 2, y0 + r) + kp;
@@ -587,10 +600,10 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
                 C Zr = mk<R>(xr_shfl(x[A - 1 - k2].x, partner), xr_shfl(x[A - 1 - k2].y, partner));
                 if (kp == 0) Zr = x[(A - k2) % A];
                 const C Zk = x[k2];
-                const C va = mk<R>((Zk.x + Zr.x) * R(0.5), (Zk.y - Zr.y) * R(0.5));
-                const C vb = mk<R>((Zk.y + Zr.y) * R(0.5), (Zr.x - Zk.x) * R(0.5));
+                const C va = mk<R>(Zk.x + Zr.x, Zk.y - Zr.y);
+                const C vb = mk<R>(Zk.y + Zr.y, Zr.x - Zk.x);
                 if (kp + B * k2 <= k1max) {
-                    const R d = dk[kp + B * k2];
+                    const R d = dk[kp + B * k2] * d3_scale;
                     if (first) o1[B * k2] = q < 3 ? mk<R>(vb.x - d * va.y, vb.y + d * va.x) : va;
                     if (second) o2[B * k2] = q == 1 ? va : vb;
                 }

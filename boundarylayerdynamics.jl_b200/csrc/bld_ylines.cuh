@@ -304,12 +304,12 @@ __global__ void __launch_bounds__((A > B ? A : B) * NL, MINB) k_fwd_yl(FwdYArgs 
             const int p = jj <= k2max ? jj : P - (K2 - jj);
             const int slot = AP == A ? p : (p / A) * AP + p % A;
             const C X = buf[slot * NL + l];
-            double vx = (double)X.x * a.inv_n, vy = (double)X.y * a.inv_n;
+            double vx = (double)X.x * a.inv_a, vy = (double)X.y * a.inv_a;
             if constexpr (SETS == 2) {
                 const C Y = buf[SB + slot * NL + l];
                 const double d = __ldg(a.d2 + jj);
-                vx += -d * ((double)Y.y * a.inv_n);
-                vy += d * ((double)Y.x * a.inv_n);
+                vx += -d * ((double)Y.y * a.inv_b);
+                vy += d * ((double)Y.x * a.inv_b);
             }
             if constexpr (MODE == 1) {
                 const double coef = ((dd1 + __ldg(a.lin.DD2 + jj)) - w.ab) - w.bc;
