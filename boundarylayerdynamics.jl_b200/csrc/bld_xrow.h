@@ -27,8 +27,10 @@ constexpr bool codelet(int n) {
 // at 84^2 x 512), else the larger A (Smagorinsky 86 / 78 us at 128^2 x 64).  A warp has
 // 32 / B lines in that pass; where that B leaves lanes idle, B = 16 takes its place if the
 // larger radix grows by no more than a third (us, before against now: advection 144
-// points single 164 / 117 at 96^2 x 512; Smagorinsky single 96 points 197 / 170, 288
-// 238 / 204, 384 284 / 263; double 160 points 274 / 253, 192 261 / 262, 224 283 / 236).
+// points single 164 / 117, double 255 / 227 at 96^2 x 512; Smagorinsky single 96 points
+// 197 / 170, 288 238 / 204, 384 284 / 263), but not for the Smagorinsky model in double
+// precision, where the larger first radix holds its own (192 points, 16 x 12 against
+// 12 x 16, 192^2 x 32 116 / 121 us).
 constexpr void factor(Shape& s, int P, bool fp32, bool adv, int multiple) {
     int best = 1 << 30;
     for (int b = 2; b <= 32; ++b) {
@@ -40,7 +42,7 @@ constexpr void factor(Shape& s, int P, bool fp32, bool adv, int multiple) {
             s.B = b;
         }
     }
-    if (!s.A || 32 % s.B == 0 || P % 16) return;
+    if (!s.A || 32 % s.B == 0 || P % 16 || !(adv || fp32)) return;
     const int a = P / 16, larger = a > 16 ? a : 16;
     if (codelet(a) && a % multiple == 0 && 3 * larger <= 4 * best) {
         s.A = a;

@@ -61,8 +61,9 @@ def test_sgs_block_kernels_do_not_spill(tmp_path):
 
 def test_row_kernel_radices(tmp_path):
     """The radices of the in-place x kernels follow from the lanes they use: a second radix
-    that leaves lanes of a warp idle has no alternative of 16 that the rule allows, and the
-    larger radix is within a third of the smallest there is.  The blocks per SM ask for no
+    that leaves lanes of a warp idle has no alternative of 16 that the rule allows (it is not
+    for the Smagorinsky model in double precision), and the larger radix is within a third of
+    the smallest there is.  The blocks per SM ask for no
     more registers than there are."""
     codelets = (2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16, 18, 24, 32)
     shapes = [line.split(",") for line in run_native(tmp_path, "row_shapes")]
@@ -74,7 +75,7 @@ def test_row_kernel_radices(tmp_path):
                  if points % q == 0 and points // q in codelets and points // q % multiple == 0]
         smallest = min(map(max, pairs))
         assert (a, b) in pairs and 3 * max(a, b) <= 4 * smallest, (kind, points, fp32, a, b)
-        if 32 % b:
+        if 32 % b and (kind == "adv" or fp32):
             assert all(q != 16 or 3 * max(p, q) > 4 * smallest for p, q in pairs), (kind, points, fp32, a, b)
         # as many registers as radix-a or radix-b values take (2 or 4 each) have to remain
         assert 65536 // (threads * blocks) >= max(a, b) * (2 if fp32 else 4), (kind, points, fp32, threads, blocks)
