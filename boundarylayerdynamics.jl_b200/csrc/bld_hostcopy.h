@@ -17,7 +17,6 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -40,8 +39,10 @@ class HostCopy {
             pin_ = nullptr;
         }
     }
-    // dev <- host or host <- dev, ordered on `st` of `device` (the current device).  On
-    // return the host array is free to change (to the device) or complete (from it).
+    // dev <- host or host <- dev, ordered on `st` of `device` (the current device).  A
+    // staged copy has read or written the whole host array when this returns, a copy that
+    // the driver was given may not have (from pinned memory it has only been enqueued), so
+    // the caller synchronises the stream before it gives the array back.
     cudaError_t copy(void* dst, const void* src, size_t bytes, bool to_device, cudaStream_t st, int device) {
         const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
         cudaPointerAttributes at{};
@@ -69,7 +70,7 @@ class HostCopy {
         int started = 1;
         try {
             for (; started < parts; ++started) threads[started] = std::thread(part, started);
-        } catch (const std::system_error&) {   // no more threads: the rest here
+        } catch (...) {   // no thread, or no memory for one: the rest here
         }
         part(0);
         for (int k = started; k < parts; ++k) part(k);

@@ -79,3 +79,8 @@ def test_row_kernel_radices(tmp_path):
             assert all(q != 16 or 3 * max(p, q) > 4 * smallest for p, q in pairs), (kind, points, fp32, a, b)
         # as many registers as radix-a or radix-b values take (2 or 4 each) have to remain
         assert 65536 // (threads * blocks) >= max(a, b) * (2 if fp32 else 4), (kind, points, fp32, threads, blocks)
+
+
+def test_host_copy_without_memory_for_threads(tmp_path):
+    """A staged copy that cannot start all its threads does their parts itself."""
+    assert run_native(tmp_path, "hostcopy_no_memory") == ["0"]
