@@ -12,6 +12,7 @@
 #include "bld_hostcopy.h"
 #include "bld_launch_util.cuh"
 #include "bld_project_tile.cuh"
+#include "bld_tune.h"
 #include "bld_yline.h"
 
 double2 h_wtab64[BLD_WTAB_SIZE];
@@ -532,8 +533,8 @@ std::vector<YCfg> y_candidates(const bld_handle* h, const Space& s, int lines_pe
     return out;
 }
 
-// average device time of `fn` after one warm-up launch, over `iters` launches or, for
-// short kernels, as many (up to 40) as take 0.2 ms: the events tick in steps of about 2 us
+// average device time of `fn` after one warm-up launch, over `iters` launches and, for
+// short kernels, once more over as many as tune_relaunches says
 template <typename F>
 int time_launches(bld_handle* h, F&& fn, int iters, float* ms) {
     cudaEvent_t e0, e1;
@@ -541,15 +542,13 @@ int time_launches(bld_handle* h, F&& fn, int iters, float* ms) {
     CUDA_TRY(cudaEventCreate(&e1));
     int st = fn();
     float t = 0;
-    for (int round = 0; round < 2 && st == BLD_OK; ++round) {
+    for (int round = 0, n = iters; round < 2 && n > 0 && st == BLD_OK; ++round, n = tune_relaunches(t, iters)) {
         if (st == BLD_OK && cudaEventRecord(e0, h->stream) != cudaSuccess) st = BLD_ERR_CUDA;
-        for (int i = 0; i < iters && st == BLD_OK; ++i) st = fn();
+        for (int i = 0; i < n && st == BLD_OK; ++i) st = fn();
         if (st == BLD_OK && cudaEventRecord(e1, h->stream) != cudaSuccess) st = BLD_ERR_CUDA;
         if (st == BLD_OK && cudaEventSynchronize(e1) != cudaSuccess) st = BLD_ERR_CUDA;
         if (st == BLD_OK) cudaEventElapsedTime(&t, e0, e1);
-        t /= iters;
-        if (t * iters >= 0.1f) break;
-        iters = std::max(iters, std::min(40, (int)(0.2f / std::max(t, 0.002f))));
+        t /= n;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

@@ -84,3 +84,12 @@ def test_row_kernel_radices(tmp_path):
 def test_host_copy_without_memory_for_threads(tmp_path):
     """A staged copy that cannot start all its threads does their parts itself."""
     assert run_native(tmp_path, "hostcopy_no_memory") == ["0"]
+
+
+def test_autotuner_launches(tmp_path):
+    """A candidate costs at most 16 launches, and a second round only where the first was
+    short and for about as long as that round has to last."""
+    rows = [tuple(map(int, line.split(","))) for line in run_native(tmp_path, "tune_launches")]
+    for us, again in rows:
+        assert 1 + 3 + again <= 16, (us, again)
+        assert again == 0 if 3 * us >= 50 else 3 <= again and again * us <= max(50, 3 * us), (us, again)
