@@ -2164,8 +2164,8 @@ int32_t bld_describe(bld_handle* h, char* buf, size_t len) {
         const char* xk = sp == 0 ? "k_adv_x" : "k_sgs_x";
         char xname[96];
         if (s.xrow)
-            snprintf(xname, sizeof xname, "%s<%s, %d, %d>", sp == 0 ? "k_adv_row" : "k_sgs_x", R, row_shape(h, s).A,
-                     row_shape(h, s).B);
+            snprintf(xname, sizeof xname, sp == 0 ? "k_adv_row<%s, %d, %d>" : "k_sgs_x<%s, %d, %d, in place>", R,
+                     row_shape(h, s).A, row_shape(h, s).B);
         else if (sp == 0 && s.x2)
             snprintf(xname, sizeof xname, "k_adv_x2<%s, %d, %d%s>", R, y2_radix_a(s.P1), y2_radix_b(s.P1),
                      s.x2 == 3 ? ", wide" : (s.x2 == 4 ? ", 2 rows" : ""));
