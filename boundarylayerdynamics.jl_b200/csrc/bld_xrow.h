@@ -9,7 +9,7 @@
 namespace bld_row {
 
 // shape of the kernel compiled for P1 = A B: rows per block, threads, blocks per SM the
-// registers are held to, forward lines in their own buffer; A = 0 where there is none
+// registers are held to, advection's forward lines in their own buffer; A = 0 where there is none
 struct Shape {
     int A = 0, B = 0, NR = 2, T = 96, MINB = 1;
     bool sepf = true;

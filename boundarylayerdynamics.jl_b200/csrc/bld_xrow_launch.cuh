@@ -28,8 +28,8 @@ cudaError_t launch_sgs_p(const XArgs& a, int nchunks, int nm, cudaStream_t st) {
     constexpr Shape s = sgs_shape(P, sizeof(R) == 4);
     if constexpr (s.A > 0) {
         static std::atomic<int> done[64];
-        const auto k = k_sgs_x<R, s.A, s.B, s.NR, s.T, s.MINB, s.sepf>;
-        const int sm = sr_smem(s.A, s.B, a.g.K1, (int)sizeof(cplx<R>), s.NR, s.sepf);
+        const auto k = k_sgs_x<R, s.A, s.B, s.NR, s.T, s.MINB>;
+        const int sm = sr_smem(s.A, s.B, a.g.K1, (int)sizeof(cplx<R>), s.NR);
         if (const cudaError_t e = opt_in(k, sm, done); e != cudaSuccess) return e;
         return bld_util::launch(k, dim3(a.P2 / s.NR, nchunks, nm), s.T, sm, st, a.overlap != 0, a);
     }

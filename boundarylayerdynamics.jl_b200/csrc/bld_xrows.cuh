@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(T, MINB) k_adv_row(XArgs a) {
 // (the halves of the two-lines-in-one unpacking), and the forward y pass takes that back.
 __host__ __device__ constexpr int sr_lines_in(int NR) { return 4 * NR + (NR + 1) / 2; }
 // dynamic shared memory: barrier, twiddles, x wavenumbers, 6 terms x NR rows, lines
-__host__ __device__ constexpr int sr_smem(int A, int B, int K1, int csz, int NR, bool sepf) {
+__host__ __device__ constexpr int sr_smem(int A, int B, int K1, int csz, int NR) {
     return 128 + xr_al(A * B * csz) + xr_al(K1 * csz / 2) + xr_al(6 * NR * K1 * csz) +
-           xr_al(sr_lines_in(NR) * xr_line(A, B) * csz) + (sepf ? xr_al(4 * NR * xr_line(A, B) * csz) : 0);
+           xr_al(sr_lines_in(NR) * xr_line(A, B) * csz) + xr_al(4 * NR * xr_line(A, B) * csz);
 }
 
 // values carried from one layer to the next at one point: velocities and strains of
@@ -415,7 +415,7 @@ __device__ __forceinline__ void sgs_row_point(const XArgs& a, const SgsLayer<R>&
 }
 
 // grid (P2 / NR, nchunks, members), block T threads; P1 = A B = 2 k1max + 2
-template <typename R, int A, int B, int NR, int T, int MINB, bool SEPF>
+template <typename R, int A, int B, int NR, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
     using C = cplx<R>;
     constexpr int P = A * B, NLI = sr_lines_in(NR), NLF = 4 * NR, LS = xr_line(A, B), BS = xr_blk(B);
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
     p += xr_al(6 * NR * K1 * csz);
     C* Ln = reinterpret_cast<C*>(p);
     p += xr_al(NLI * LS * csz);
-    C* Fw = SEPF ? reinterpret_cast<C*>(p) : Ln;
+    C* Fw = reinterpret_cast<C*>(p);   // the forward lines have a buffer of their own
     const C* Min = reinterpret_cast<const C*>(a.min) + (long long)m * a.min_mstride;
     C* Mout = reinterpret_cast<C*>(a.mout) + (long long)m * a.mout_mstride;
     const double* lcm = a.lc + (long long)m * n3;
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
                 xr_block<R, A, B, +1>(Ln + L * LS + q * BS, tw, q);
             }
             __syncthreads();
-        } else if (SEPF) {
+        } else {
             __syncthreads();   // the forward lines of the layer below have been read
         }
         const int c = j - 1;   // C layer completed at this step
@@ -609,7 +609,6 @@ __global__ void __launch_bounds__(T, MINB) k_sgs_x(XArgs a) {
                 }
             }
         }
-        if (!SEPF) __syncthreads();
     }
 }
 
