@@ -12,7 +12,7 @@ from conftest import PKG_DIR
 
 CSRC = os.path.join(PKG_DIR, "csrc")
 # tables of a handle, written when it is created
-TABLES = r"a\.(lin\.)?(d1|d2|DD1|DD2|alpha_c|alpha_i|inv_alpha_c)\b"
+TABLES = r"a\.(lin\.)?(d1|d2|DD1|DD2|(inv_|d3_)?alpha_c|(d3_)?alpha_i)\b"
 # the state in the epilogue of k_fwd_yl
 COMPLETE = {"bld_ylines.cuh": r"S[0z] \+"}
 
