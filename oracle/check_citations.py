@@ -18,7 +18,9 @@ import re
 import sys
 
 REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-DEFAULT_REF = "/root/reference"
+MOUNT = "/root/reference"
+# the checkout, or where its sources would be if the mount point is empty (no directory)
+DEFAULT_REF = MOUNT if os.path.isdir(os.path.join(MOUNT, "src")) else os.path.join(MOUNT, "src")
 CITE = re.compile(r"\b((?:src|test|docs|benchmark)/[A-Za-z0-9_./-]+\.(?:jl|md|toml)):(\d+(?:-\d+)?(?:,\d+(?:-\d+)?)*)")
 # this repository's own sources: the package, the kernels, the header, the
 # oracle, the tests, the bench and entry points, and the design and integration notes
