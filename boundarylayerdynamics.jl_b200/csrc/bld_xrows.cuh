@@ -27,9 +27,9 @@
 // leave two to eight independent blocks per SM, four barriers per layer instead of
 // five, and no spectra in shared memory.  Measured (us per launch, before -> now):
 // advection 192^2 x 96 double 238 -> 181, single 130 -> 99; 512^2 x 64 single
-// 944 -> 466; 128^2 x 64 single 45 -> 35; Smagorinsky 256^2 x 64 double 584 -> 281,
+// 944 -> 466; 128^2 x 64 single 45 -> 35; Smagorinsky 256^2 x 64 double 584 -> 287,
 // 512^2 x 64 single 920 -> 600, 128^2 x 64 single 71 -> 47.  Now shared-memory
-// wavefronts (55 to 65 % of peak) and issue slots (37 to 58 %) share the time.
+// wavefronts (48 to 64 % of peak) and issue slots (32 to 62 %) share the time.
 #pragma once
 
 #include "bld_dft.cuh"

@@ -18,8 +18,8 @@
 // the more warps are resident the better, so the registers are held as low as the larger
 // radix allows.  The forward epilogue took two thirds of that pass's instructions.
 // Measured (us per launch, k_inv_y2 / k_fwd_y2 -> here): inverse 512^2 x 32 single
-// 768 points 186 -> 168, 128^2 x 256 single 192 points 81 -> 70, 192^2 x 96 288 points
-// single 70 -> 64, double 104 -> 102, 128^2 x 512 double 128 points 156 -> 136; forward
+// 768 points 186 -> 162, 128^2 x 256 single 192 points 81 -> 66, 192^2 x 96 288 points
+// single 70 -> 62, double 104 -> 100, 128^2 x 512 double 128 points 156 -> 136; forward
 // 192^2 x 96 288 points double 153 -> 107, single 113 -> 79; 512^2 x 32 single
 // 768 points 237 -> 180, 512 points with two line sets 277 -> 239; 128^2 x 256 single
 // 192 points 113 -> 76.
