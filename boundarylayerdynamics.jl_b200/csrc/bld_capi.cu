@@ -905,6 +905,8 @@ int autotune_impl(bld_handle* h) {
         const int only_t = (pt && pt[0]) ? atoi(pt) : -1;
         const char* pp = getenv("BLD_PROJ_PIPE");
         const int only_p = (pp && pp[0]) ? atoi(pp) : -1;
+        int nsm = 0;
+        CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
         float bt = 1e30f;
         int btile = 0, bpipe = 0;
         for (int ln : {0, 4, 8, 16})
@@ -912,6 +914,8 @@ int autotune_impl(bld_handle* h) {
                 if (ln && !project_tile_ok(h, ln)) continue;
                 if (pipe && (!ln || !project_pipe_ok(h, ln))) continue;
                 if (only_t >= 0 && ln != only_t) continue;
+                // with no more tiles than SMs a persistent block has one tile, as a plain one
+                if (pipe && only_p != 1 && (h->g.F + ln - 1) / ln * (long long)B <= nsm) continue;
                 // a forced persistent form that does not fit keeps the plain one
                 if (ln && only_p >= 0 && pipe != only_p && !(only_p == 1 && !project_pipe_ok(h, ln))) continue;
                 h->proj_tile = ln;
